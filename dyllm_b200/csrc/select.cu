@@ -4,11 +4,14 @@
 //   context_stats   reads 2 * width * 2 bytes per row, writes 12
 //   cosine_mask     reads 12 bytes per row, writes 1
 //   salient_select  reads 12 bytes per row once, writes 8 (+4, +8) bytes per selected row
+#include <cooperative_groups.h>
+
 #include <atomic>
 
 #include "common.cuh"
 
 namespace dyllm {
+namespace cg = cooperative_groups;
 namespace {
 
 // ----------------------------------------------------------------------------------------------
@@ -97,10 +100,13 @@ __global__ void cosine_mask_kernel(const float* __restrict__ stats, uint8_t* __r
 }
 
 // ----------------------------------------------------------------------------------------------
-// salient_select: warp-ballot flags + block scan + decoupled look-back across tiles
+// salient_select: flags + warp and block scans + counts exchanged between the CTAs
 // ----------------------------------------------------------------------------------------------
 constexpr int kSelWarps = 8;
-constexpr int kSelTileRowsSmall = kSelWarps * 2 * 128;   // 2048 rows per tile (workspace is sized for these)
+constexpr int kSelTileRowsSmall = kSelWarps * 2 * 128;   // 2048 rows (the workspace holds one descriptor for each)
+constexpr int kSelClusterWarps = 16;
+constexpr int kSelClusterCtas = 8;
+constexpr int kSelClusterRows = kSelClusterCtas * kSelClusterWarps * 128;   // rows of a cluster per 128-row group of a warp
 constexpr uint32_t kLookbackSpinLimit = 1u << 24;
 
 // Workspace layout: [0] ticket counter (uint32), [1] padding, then one 64-bit descriptor per tile:
@@ -123,37 +129,37 @@ __device__ __forceinline__ int lower_bound_i32(const int32_t* a, int n, int key)
   return lo;
 }
 
-// Each thread owns 4 consecutive rows of a 128-row group (48 contiguous bytes = three 16-byte loads),
-// so a warp reads 1536 contiguous bytes per group; a warp takes SUPER groups, a tile 8 * SUPER * 128
-// rows.  Flags become a 4-bit nibble per thread; positions come from a warp prefix sum of the nibble
-// popcounts, a block scan over the warps and a decoupled look-back over the tiles (32 predecessors per
-// step).  The prefix front moves a bounded number of tiles per microsecond, which is what small inputs
-// (up to 64 Ki rows, SUPER = 2) want: many small tiles in flight.  Larger inputs take
-// salient_select_ranges_kernel below.
+// Each thread owns 4 consecutive rows of a 128-row group (48 contiguous bytes = three 16-byte loads), so a warp reads
+// 1536 contiguous bytes per group; a warp takes SUPER groups, a CTA 16 * SUPER * 128 rows.  Flags become a 4-bit nibble
+// per thread; positions come from a warp prefix sum of the nibble popcounts, a block scan over the warps, and the counts
+// of the CTAs before this one, which the (at most eight) CTAs of the one cluster hand each other through distributed
+// shared memory.  Up to 64 Ki rows (every step of the package's workloads), where the launch is bound by latency: no
+// scratch memory, so no clearing of it either.  (The chained look-back that this replaced needed a zeroed workspace;
+// inside a captured step the memset node and the switches to and from it took 9 us between the kernels on both sides,
+// the selection itself 7.6 us at 8192 rows.)  SUPER = 1 up to 16 Ki rows spreads the loads over more SMs; 4 beyond.
+// Larger inputs take salient_select_ranges_kernel below.
 template <int SUPER>
-__global__ void __launch_bounds__(kSelWarps * 32)
+__global__ void __launch_bounds__(kSelClusterWarps * 32)
 salient_select_kernel(const float* __restrict__ stats, int rows, float threshold,
                       const int32_t* __restrict__ cu_seqlens_q, int batch, const int32_t* __restrict__ cu_promptlens,
                       int64_t* __restrict__ idx_out, int32_t* __restrict__ idx32_out, int64_t* __restrict__ idx_k_out,
                       int32_t* __restrict__ cu_salientlens_out, int32_t* __restrict__ count_out,
-                      uint8_t* __restrict__ mask_out, SelectWorkspace* ws, int* status_word) {
+                      uint8_t* __restrict__ mask_out) {
   pdl_wait();      // programmatic dependent launch: nothing before this reads an earlier kernel's data
   pdl_trigger();
-  constexpr int kTileRows = kSelWarps * SUPER * 128;
-  __shared__ int s_excl[kSelWarps * SUPER * 32];       // per thread and group: flags of the tile before its rows
-  __shared__ uint8_t s_nib[kSelWarps * SUPER * 32];    // per thread and group: its 4 flags
-  __shared__ int s_warp_count[kSelWarps];
-  __shared__ int s_tile;
-  __shared__ int s_tile_prefix;
+  constexpr int kTileRows = kSelClusterWarps * SUPER * 128;
+  __shared__ int s_excl[kSelClusterWarps * SUPER * 32];       // per thread and group: flags of the tile before its rows
+  __shared__ uint8_t s_nib[kSelClusterWarps * SUPER * 32];    // per thread and group: its 4 flags
+  __shared__ int s_warp_count[kSelClusterWarps];
+  __shared__ int s_cta_count[kSelClusterCtas];
   __shared__ int s_b_range[2];
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();      // awaited before the first access to another CTA's shared memory: all have started
 
-  if (threadIdx.x == 0)
-    s_tile = static_cast<int>(atomicAdd(&ws->ticket, 1u));
-  __syncthreads();
-  const int tile = s_tile;
+  const int tile = blockIdx.x;   // the grid is one cluster
   const int tile_row0 = tile * kTileRows;
   const int tile_row1 = min(tile_row0 + kTileRows, rows);
   // sequence boundaries inside this tile: two binary searches by two threads, under the loads below
@@ -222,58 +228,20 @@ salient_select_kernel(const float* __restrict__ stats, int rows, float threshold
     s_warp_count[warp] = warp_count;
   __syncthreads();
 
-  // 2. tile aggregate, then exclusive prefix over earlier tiles: decoupled look-back by warp 0, whose
-  // 32 lanes inspect 32 predecessors at a time
+  // 2. this CTA's count to every CTA of the cluster, then the sum of those before it
+  cluster.barrier_wait();
   if (warp == 0) {
-    int t = lane < kSelWarps ? s_warp_count[lane] : 0;
+    int t = lane < kSelClusterWarps ? s_warp_count[lane] : 0;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
       t += __shfl_xor_sync(0xffffffffu, t, off);
-    const int aggregate = t;
-    volatile unsigned long long* tiles = ws->tiles;
-    if (lane == 0) {
-      tiles[tile] = ((tile == 0 ? 2ull : 1ull) << 32) | static_cast<unsigned int>(aggregate);
-      __threadfence();
-    }
-    int exclusive = 0;
-    bool gave_up = false;
-    for (int base = tile - 1; base >= 0 && !gave_up; base -= 32) {
-      const int look = base - lane;
-      unsigned long long d = 2ull << 32;   // before the first tile: inclusive prefix 0
-      uint32_t spins = 0;
-      for (;;) {
-        if (look >= 0)
-          d = tiles[look];
-        const bool ready = ((d >> 32) & 3ull) != 0;
-        if (__all_sync(0xffffffffu, ready))
-          break;
-        if (++spins > kLookbackSpinLimit) {
-          gave_up = true;
-          break;
-        }
-      }
-      gave_up = __any_sync(0xffffffffu, gave_up);
-      const uint32_t inclusive_mask = __ballot_sync(0xffffffffu, ((d >> 32) & 3ull) == 2);
-      const int first = inclusive_mask ? __ffs(inclusive_mask) - 1 : 31;   // nearest predecessor with a full prefix
-      int contrib = lane <= first ? static_cast<int>(static_cast<unsigned int>(d)) : 0;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-        contrib += __shfl_xor_sync(0xffffffffu, contrib, off);
-      exclusive += contrib;
-      if (inclusive_mask)
-        break;
-    }
-    if (lane == 0) {
-      if (gave_up && status_word)
-        atomicCAS(status_word, 0, 101);
-      if (tile != 0)
-        tiles[tile] = (2ull << 32) | static_cast<unsigned int>(exclusive + aggregate);
-      __threadfence();
-      s_tile_prefix = exclusive;
-    }
+    if (lane < static_cast<int>(gridDim.x))
+      *cluster.map_shared_rank(&s_cta_count[tile], lane) = t;
   }
-  __syncthreads();
-  const int tile_prefix = s_tile_prefix;
+  cluster.sync();   // the last access to another CTA's shared memory: CTAs may end on their own after it
+  int tile_prefix = 0;
+  for (int t = 0; t < tile; ++t)
+    tile_prefix += s_cta_count[t];
 
   // 3. ordered writes
   int base = tile_prefix;
@@ -314,7 +282,7 @@ salient_select_kernel(const float* __restrict__ stats, int rows, float threshold
   }
   if (tile_row1 == rows) {  // last tile: boundaries at or beyond the end, and the total
     int total = tile_prefix;
-    for (int w = 0; w < kSelWarps; ++w)
+    for (int w = 0; w < kSelClusterWarps; ++w)
       total += s_warp_count[w];
     for (int b = b_hi + threadIdx.x; b <= batch; b += blockDim.x)
       cu_salientlens_out[b] = total;
@@ -587,24 +555,30 @@ int launch_salient_select(const float* stats, int rows, float threshold, const i
     DYLLM_LAUNCH(select_empty_kernel, 1, 128, 0, stream, cu_salientlens_out, count_out, batch);
     return check_launch("salient_select(empty)");
   }
+  if (rows <= 4 * kSelClusterRows) {
+    if (rows <= kSelClusterRows)
+      launch_pdl_cluster(salient_select_kernel<1>, cdiv_i(rows, kSelClusterWarps * 128), kSelClusterWarps * 32, 0, stream,
+                         cdiv_i(rows, kSelClusterWarps * 128), stats, rows, threshold, cu_seqlens_q, batch, cu_promptlens,
+                         idx_out, idx32_out, idx_k_out, cu_salientlens_out, count_out, mask_out);
+    else
+      launch_pdl_cluster(salient_select_kernel<4>, cdiv_i(rows, kSelClusterWarps * 512), kSelClusterWarps * 32, 0, stream,
+                         cdiv_i(rows, kSelClusterWarps * 512), stats, rows, threshold, cu_seqlens_q, batch, cu_promptlens,
+                         idx_out, idx32_out, idx_k_out, cu_salientlens_out, count_out, mask_out);
+    return check_launch("salient_select");
+  }
   if (cudaMemsetAsync(workspace, 0, select_workspace_bytes(rows), stream) != cudaSuccess)
     return set_error(DYLLM_ERR_CUDA, "salient_select: clearing the workspace failed");
   SelectWorkspace* w = static_cast<SelectWorkspace*>(workspace);
-  if (rows > 64 * 1024) {
-    // contiguous ranges, one per CTA the device runs at once (four per SM: 63 registers, 18 KB of shared memory)
-    const int64_t resident = 4ll * sm_count();
-    int64_t per = (static_cast<int64_t>(rows) + resident - 1) / resident;
-    per = (per + 127) / 128 * 128;   // whole 128-row groups; the ranges stay balanced over the SMs
-    per = per < kSelTileRowsSmall ? kSelTileRowsSmall : per;   // the workspace holds one descriptor per 2048 rows
-    per = per > kRangeMaxRows ? kRangeMaxRows : per;
-    const int rows_per_cta = static_cast<int>(per);
-    DYLLM_LAUNCH(salient_select_ranges_kernel, cdiv_i(rows, rows_per_cta), kSelWarps * 32, 0, stream,
-        stats, rows, threshold, cu_seqlens_q, batch, cu_promptlens, idx_out, idx32_out, idx_k_out,
-        cu_salientlens_out, count_out, mask_out, w, rows_per_cta, device_status_word());
-  } else
-    DYLLM_LAUNCH(salient_select_kernel<2>, cdiv_i(rows, kSelTileRowsSmall), kSelWarps * 32, 0, stream, 
-        stats, rows, threshold, cu_seqlens_q, batch, cu_promptlens, idx_out, idx32_out, idx_k_out,
-        cu_salientlens_out, count_out, mask_out, w, device_status_word());
+  // contiguous ranges, one per CTA the device runs at once (four per SM: 63 registers, 18 KB of shared memory)
+  const int64_t resident = 4ll * sm_count();
+  int64_t per = (static_cast<int64_t>(rows) + resident - 1) / resident;
+  per = (per + 127) / 128 * 128;   // whole 128-row groups; the ranges stay balanced over the SMs
+  per = per < kSelTileRowsSmall ? kSelTileRowsSmall : per;   // the workspace holds one descriptor per 2048 rows
+  per = per > kRangeMaxRows ? kRangeMaxRows : per;
+  const int rows_per_cta = static_cast<int>(per);
+  DYLLM_LAUNCH(salient_select_ranges_kernel, cdiv_i(rows, rows_per_cta), kSelWarps * 32, 0, stream,
+      stats, rows, threshold, cu_seqlens_q, batch, cu_promptlens, idx_out, idx32_out, idx_k_out,
+      cu_salientlens_out, count_out, mask_out, w, rows_per_cta, device_status_word());
   return check_launch("salient_select");
 }
 
