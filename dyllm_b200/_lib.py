@@ -36,6 +36,7 @@ SIGNATURES: dict[str, tuple] = {
     "dyllm_cache_scatter_update": (I, [P, P, P, P, I, P, P, I, I, P, I, I, P]),
     "dyllm_gathered_linear_workspace_bytes": (Z, [I, I, I]),
     "dyllm_gathered_linear": (I, [P, I, I, c_int64, P, I, P, I, P, I, P, c_int64, P, c_int64, I, P, P, P, Z, I, I, P]),
+    "dyllm_gathered_linear_bias": (I, [P, I, I, c_int64, P, I, P, I, P, I, P, c_int64, P, c_int64, I, P, P, P, Z, I, I, P, I, P]),
     "dyllm_swiglu_ffn_workspace_bytes": (Z, [I, I, I]),
     "dyllm_swiglu_ffn": (I, [P, I, I, c_int64, P, I, P, I, P, P, I, P, c_int64, P, P, Z, I, I, P]),
     "dyllm_cache_dest_rows": (I, [P, P, P, P, I, I, P, P, P]),
@@ -81,7 +82,7 @@ KERNELS_PER_CALL = {
     "dyllm_context_stats": 1, "dyllm_cosine_mask": 1, "dyllm_salient_select": 1, "dyllm_salient_select_static": 1,
     "dyllm_fused_offset": 1,
     "dyllm_cache_get_seqs": 1, "dyllm_cache_get_block": 1, "dyllm_cache_reset_full": 1, "dyllm_cache_reset_block": 1,
-    "dyllm_cache_scatter_update": 1, "dyllm_gathered_linear": 2, "dyllm_swiglu_ffn": 3, "dyllm_cache_dest_rows": 1, "dyllm_moe_route": 1, "dyllm_moe_ffn": 5,
+    "dyllm_cache_scatter_update": 1, "dyllm_gathered_linear": 2, "dyllm_gathered_linear_bias": 2, "dyllm_swiglu_ffn": 3, "dyllm_cache_dest_rows": 1, "dyllm_moe_route": 1, "dyllm_moe_ffn": 5,
     "dyllm_attention_sparse_varlen": 2, "dyllm_attention_salient_rows": 2, "dyllm_delta_v_update": 1,
     "dyllm_add_rms_norm": 1, "dyllm_add_rms_norm_segmented": 1, "dyllm_add_rms_norm_rows": 1, "dyllm_head_rms_norm": 1, "dyllm_rope_neox": 1, "dyllm_row_confidence": 1, "dyllm_confidence_unmask": 1, "dyllm_kv_cache_update": 1,
     "dyllm_tp_push_rows": 1, "dyllm_tp_reduce_rows": 1, "dyllm_tp_allreduce_rows": 2, "dyllm_tp_push_f32": 1,

@@ -1,18 +1,16 @@
 // Gathered linear layers and the SwiGLU FFN on salient rows:
 //   out[map[m]] = down( silu(x[idx[m]] Wg^T) * (x[idx[m]] Wu^T) )
-// built from the tcgen05 GEMM in gemm.cuh: gate/up with the activation fused in the epilogue, then the
-// down projection whose epilogue scatters rows to their destination.  Activation rows reach the GEMM
-// either through a small staging copy (rows gathered once into a compact buffer, then plain TMA boxes)
-// or directly by TMA gather4.  Launch shapes are chosen from a row-count hint; the live row count is
-// read on the device, so no host synchronisation is needed.
+// built from two tcgen05 GEMMs: gate/up with the activation fused in the epilogue, then the down projection
+// whose epilogue scatters rows to their destination.  By default the rows are packed (by the caller, or by a
+// small staging copy) and run on the CTA-pair GEMM of pair_gemm.cuh, which suits every row count.  Calls that
+// name a tile width or ask for TMA gather4 run on gemm.cuh, whose launch shape follows a row-count hint.  The
+// live row count is read on the device, so no host synchronisation is needed.
 #include <atomic>
 
 #include "gemm.cuh"
+#include "pair_gemm.cuh"
 
 namespace dyllm {
-
-constexpr int kSplitRows = 512;   // split-K partial sums are kept for at most this many live rows
-constexpr int kMaxSplits = 4;
 
 namespace {
 
@@ -120,6 +118,23 @@ Plan make_plan(bool swiglu, int M, int hint, int n, int K, int tile_n, bool can_
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// Which of the two kernels runs a call that names neither a tile width nor a_mode 1 (both give the same bits).  The pair
+// kernel needs no row estimate and wins almost everywhere; its tiles are 256 columns per pair of SMs, so narrow or short
+// products of few rows leave it with too few of them, where 64-column tiles still fill SMs (us, 64-column : pair kernel):
+//   gate/up of 1536 columns, 46 / 300 rows            30 : 35 / 31 : 47
+//   plain, 1024 columns, 46 / 100 rows                13 : 16 / 16 : 17
+//   plain, K = 1536, 4096 columns, 46 / 100 rows      12 : 14 / 15 : 17
+//   gate/up of 12288 columns, 65 .. 128 rows          43 : 48  (46 rows 41 : 42, 160 rows 70 : 50; only when the host
+//                                                     knows the count: one estimate serves every count otherwise)
+bool few_tiles(bool swiglu, int n, int K, int num_rows, const int32_t* num_rows_dev, int rows_hint) {
+  const int h = rows_hint > 0 && rows_hint < num_rows ? rows_hint : num_rows;
+  if (h > kSplitRows)
+    return false;
+  if (swiglu)
+    return n < 6144 || (!num_rows_dev && num_rows > 64 && num_rows <= 128);
+  return n <= 2048 || K < 2048;
+}
+
 size_t padded_rows(int rows) { return static_cast<size_t>(cdiv_i(rows, kGemmBM)) * kGemmBM; }
 
 // dest[m] = seq_starts[seq_ids[b]] + (row_idx[m] - cu[b]) for m < n, -1 beyond the live rows.
@@ -171,7 +186,7 @@ int launch_gathered_gemm(bool swiglu, int a_mode, int tile_n, const GemmParams& 
   if (p.M <= 0)
     return DYLLM_OK;
   const Plan plan = make_plan(swiglu, p.M, rows_hint, n, p.K, tile_n, partial != nullptr,
-                              a_mode == 0 && !p.tile_expert);
+                              a_mode == 0);
   DYLLM_REQUIRE((plan.tile_n == 64 || plan.tile_n == 128 || (plan.tile_n == 256 && plan.tall && !swiglu)) &&
                     n % plan.tile_n == 0,
                 DYLLM_ERR_UNSUPPORTED,
@@ -274,6 +289,16 @@ int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ld
                           int64_t ldo, void* out2, int64_t ldo2, int split_col, const int32_t* out_row_map,
                           const float* row_scale, void* workspace, size_t workspace_bytes, int a_mode, int tile_n,
                           void* stream) {
+  return dyllm_gathered_linear_bias(x, x_rows, in_features, ldx, idx, num_rows, num_rows_dev, rows_hint, weight,
+                                      out_features, out, ldo, out2, ldo2, split_col, out_row_map, row_scale, workspace,
+                                      workspace_bytes, a_mode, tile_n, nullptr, 0, stream);
+}
+
+int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64_t ldx, const int32_t* idx,
+                                 int num_rows, const int32_t* num_rows_dev, int rows_hint, const void* weight,
+                                 int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
+                                 const int32_t* out_row_map, const float* row_scale, void* workspace,
+                                 size_t workspace_bytes, int a_mode, int tile_n, const void* bias, int few_rows_ctas, void* stream) {
   DYLLM_REQUIRE(x_rows >= 0 && in_features > 0 && out_features > 0 && num_rows >= 0, DYLLM_ERR_INVALID_ARGUMENT,
                 "gathered_linear: x_rows %d in %d out %d num_rows %d", x_rows, in_features, out_features, num_rows);
   if (num_rows == 0 || x_rows == 0)
@@ -298,6 +323,9 @@ int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ld
   g.a_rows = x_rows;
   int64_t lda = ldx;
   int mode = a_mode;
+  DYLLM_REQUIRE(!bias || (mode == 0 && tile_n == 0), DYLLM_ERR_UNSUPPORTED,
+                "gathered_linear: a bias needs a_mode 0 and no tile width");
+  DYLLM_REQUIRE(few_rows_ctas >= 0, DYLLM_ERR_INVALID_ARGUMENT, "gathered_linear: few_rows_ctas %d", few_rows_ctas);
   if (idx && a_mode == 0) {
     int rc = stage_rows(x, ldx, idx, x_rows, workspace, in_features, num_rows, num_rows_dev, rows_hint, s);
     if (rc != DYLLM_OK)
@@ -313,7 +341,6 @@ int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ld
   g.m_count_dev = num_rows_dev;
   g.M = num_rows;
   g.K = in_features;
-  g.b_rows_per_expert = out_features;
   g.out = static_cast<__nv_bfloat16*>(out);
   g.ldc = ldo;
   g.out2 = static_cast<__nv_bfloat16*>(out2);
@@ -322,6 +349,24 @@ int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ld
   g.out_row_map = out_row_map;
   g.row_scale = row_scale;
   float* partial = have_ws ? reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + stage_bytes) : nullptr;
+  if (bias || (mode == 0 && tile_n == 0 && !few_tiles(false, out_features, in_features, num_rows, num_rows_dev, rows_hint))) {
+    PairGemmParams q = {};
+    q.m_count_dev = num_rows_dev;
+    q.M = num_rows;
+    q.K = in_features;
+    q.n = out_features;
+    q.out = g.out;
+    q.ldc = ldo;
+    q.out2 = g.out2;
+    q.ldc2 = g.ldc2;
+    q.split_col = g.split_col;
+    q.out_row_map = out_row_map;
+    q.row_scale = row_scale;
+    q.bias = static_cast<const __nv_bfloat16*>(bias);
+    q.partial = partial;
+    q.one_tile_pairs = few_rows_ctas > 0 ? (few_rows_ctas + 1) / 2 : 0;
+    return launch_pair_gemm(false, q, g.a, g.a_rows, lda, weight, out_features, s);
+  }
   return launch_gathered_gemm(false, mode, tile_n, g, lda, weight, out_features, out_features, rows_hint, partial, s);
 }
 
@@ -368,25 +413,47 @@ int dyllm_swiglu_ffn(const void* x, int x_rows, int hidden, int64_t ldx, const i
   } else {
     mode = 0;
   }
-  g1.m_count_dev = num_rows_dev;
-  g1.M = num_rows;
-  g1.K = hidden;
-  g1.b_rows_per_expert = 2 * inter;
-  g1.up_row_offset = inter;
-  g1.out = reinterpret_cast<__nv_bfloat16*>(inter_buf);
-  g1.ldc = inter;
-  int rc = launch_gathered_gemm(true, mode, tile_n, g1, lda, w_gate_up, 2 * static_cast<int64_t>(inter), inter,
-                                rows_hint, nullptr, s);
+  PairGemmParams q = {};
+  q.m_count_dev = num_rows_dev;
+  q.M = num_rows;
+  q.partial = partial;
+  const bool choose = mode == 0 && tile_n == 0;
+  int rc;
+  if (choose && !few_tiles(true, inter, hidden, num_rows, num_rows_dev, rows_hint)) {
+    q.K = hidden;
+    q.n = inter;
+    q.up_row_offset = inter;
+    q.out = reinterpret_cast<__nv_bfloat16*>(inter_buf);
+    q.ldc = inter;
+    rc = launch_pair_gemm(true, q, g1.a, g1.a_rows, lda, w_gate_up, 2 * static_cast<int64_t>(inter), s);
+  } else {
+    g1.m_count_dev = num_rows_dev;
+    g1.M = num_rows;
+    g1.K = hidden;
+    g1.up_row_offset = inter;
+    g1.out = reinterpret_cast<__nv_bfloat16*>(inter_buf);
+    g1.ldc = inter;
+    rc = launch_gathered_gemm(true, mode, tile_n, g1, lda, w_gate_up, 2 * static_cast<int64_t>(inter), inter, rows_hint,
+                              nullptr, s);
+  }
   if (rc != DYLLM_OK)
     return rc;
 
+  if (choose && !few_tiles(false, hidden, inter, num_rows, num_rows_dev, rows_hint)) {
+    q.K = inter;
+    q.n = hidden;
+    q.up_row_offset = 0;
+    q.out = static_cast<__nv_bfloat16*>(out);
+    q.ldc = ldo;
+    q.out_row_map = out_row_map;
+    return launch_pair_gemm(false, q, inter_buf, static_cast<int>(padded), inter, w_down, hidden, s);
+  }
   GemmParams g2 = {};
   g2.a = reinterpret_cast<const __nv_bfloat16*>(inter_buf);
   g2.m_count_dev = num_rows_dev;
   g2.M = num_rows;
   g2.K = inter;
   g2.a_rows = static_cast<int>(padded);
-  g2.b_rows_per_expert = hidden;
   g2.out = static_cast<__nv_bfloat16*>(out);
   g2.ldc = ldo;
   g2.out_row_map = out_row_map;

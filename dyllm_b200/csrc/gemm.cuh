@@ -1,7 +1,8 @@
-// Row-gathered bf16 GEMM on the 5th-generation tensor cores (tcgen05 + TMEM), shared by the dense
-// SwiGLU FFN, the K/V projection of salient rows and the MoE expert FFN.
+// Row-gathered bf16 GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for the dense SwiGLU FFN and the K/V
+// projection of salient rows: the calls that name a tile width or TMA gather4, and products of few rows with few columns
+// (few_tiles() in ffn.cu); everything else runs on pair_gemm.cuh.
 //
-//   D[m, n] = sum_k A[a_idx[m], k] * B[b_row0(m_tile) + n, k]          (fp32 accumulation in TMEM)
+//   D[m, n] = sum_k A[a_idx[m], k] * B[n, k]                           (fp32 accumulation in TMEM)
 //
 // The number of live rows is read on the device (m_count_dev), so a launch needs no host knowledge of
 // it: the grid is (n tiles, k splits, row groups) and every CTA walks over the row tiles
@@ -27,11 +28,9 @@ struct GemmParams {
   const __nv_bfloat16* a;      // activation matrix
   const int32_t* a_idx;        // [M] source row of A for logical row m (A_MODE 1); null = identity
   const int32_t* m_count_dev;  // device scalar bounding the live logical rows; null = M
-  const int32_t* tile_expert;  // [ceil(M/128)] weight block per row tile; null = block 0
   int M;                       // upper bound of logical rows
   int K;                       // contraction length, multiple of 64
   int a_rows;                  // rows of the activation matrix (for clamping)
-  int b_rows_per_expert;       // rows of B per weight block
   int up_row_offset;           // SwiGLU: row distance from the gate rows to the up rows
   __nv_bfloat16* out;          // output matrix
   int64_t ldc;                 // row pitch of the output in elements
@@ -166,7 +165,7 @@ gathered_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     int it = 0;
     for (int mt = blockIdx.z; mt * BM < m_count; mt += gridDim.z) {
       const int m0 = mt * BM;
-      const int b_row0 = (p.tile_expert ? p.tile_expert[mt] : 0) * p.b_rows_per_expert + n_tile * BNH;
+      const int b_row0 = n_tile * BNH;
       int rows4[4] = {0, 0, 0, 0};
       if (A_MODE == 1) {
 #pragma unroll

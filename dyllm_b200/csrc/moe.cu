@@ -1,20 +1,16 @@
 // Mixture-of-experts FFN on salient rows: softmax top-k router, expert-sorted grouped GEMMs on the
-// tcgen05 kernel of gemm.cuh (one weight block per 128-row tile), routing weight folded into the
+// CTA-pair kernel of pair_gemm.cuh (one weight block per row tile), routing weight folded into the
 // down-projection epilogue, per-token sum over the top-k slots.
 //
 //   route    logits = x[idx[m]] . Wr^T (fp32), softmax over experts, top-k           (one block per row)
-//   align    (row, slot) pairs grouped by expert, every group padded to 128 rows  (one block)
+//   align    (row, slot) pairs grouped by expert, row tiles of at most 256 rows  (one block)
 //   GEMM 1   h = silu(x Wg_e^T) * (x Wu_e^T) for the rows of each tile's expert
 //   GEMM 2   y[pair] = w_pair * (h Wd_e^T)
 //   combine  out[map[m]] = sum over the owned slots of row m of y[m * k + j]
 #include "gemm.cuh"
+#include "pair_gemm.cuh"
 
 namespace dyllm {
-
-int launch_gathered_gemm(bool swiglu, int a_mode, int tile_n, const GemmParams& p_in, int64_t lda, const void* b,
-                         int64_t b_total_rows, int n, int rows_hint, float* partial, cudaStream_t stream);
-int stage_rows(const void* x, int64_t ldx, const int32_t* idx, int x_rows, void* compact, int width, int num_rows,
-               const int32_t* num_rows_dev, int rows_hint, cudaStream_t stream);
 
 namespace {
 
@@ -117,63 +113,160 @@ moe_route_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t
   }
 }
 
-// Single block: groups the owned (row, slot) pairs by local expert, pads every group to 128 rows and
-// writes, per padded position, the source row, the destination pair and the routing weight.
-__global__ void __launch_bounds__(1024)
-moe_align_kernel(const int32_t* __restrict__ topk_ids, const float* __restrict__ topk_w, int num_rows,
+// Single block: the position of every owned (row, slot) pair when the pairs are grouped by local expert, in pair order
+// inside an expert (-1 for a pair of another rank's expert), and the row tiles of every expert (at most 256 rows each,
+// spread evenly in steps of 32: the tiles of pair_gemm.cuh).  Every warp owns a contiguous part of the pairs and counts
+// it with warp matches, so no counter is shared between warps and the order is the same in every run.  Only the positions
+// are written here, coalesced; what lies at a position is scattered by moe_stage_kernel on all SMs (from this one SM the
+// scattered stores alone took 25 of 35 us at 24 000 pairs).
+constexpr int kAlignWarps = 32;
+constexpr int kAlignBatch = 8;   // independent loads in flight per lane
+
+__global__ void __launch_bounds__(kAlignWarps * 32)
+moe_align_kernel(const int32_t* __restrict__ topk_ids, int num_rows,
                  const int32_t* __restrict__ num_rows_dev, int top_k, int expert_start, int num_local_experts,
-                 const int32_t* __restrict__ row_src, int32_t* __restrict__ a_idx, int32_t* __restrict__ pair_idx,
-                 float* __restrict__ pair_w, int32_t* __restrict__ tile_expert, int32_t* __restrict__ m_total,
-                 int capacity) {
+                 int32_t* __restrict__ pair_pos, int4* __restrict__ row_tiles, int32_t* __restrict__ tiles_dev) {
   pdl_wait();      // programmatic dependent launch: nothing before this reads an earlier kernel's data
   pdl_trigger();
-  __shared__ int s_count[kMaxExperts];
-  __shared__ int s_start[kMaxExperts + 1];
-  __shared__ int s_fill[kMaxExperts];
+  __shared__ int s_next[kAlignWarps][kMaxExperts];   // pairs per warp and expert, then the warp's next position
+  __shared__ int s_warp[2][kMaxExperts / 32];
+  __shared__ int s_max;
   const int n = num_rows_dev ? min(num_rows, *num_rows_dev) : num_rows;
   const int pairs = n * top_k;
-  for (int e = threadIdx.x; e < num_local_experts; e += blockDim.x) {
-    s_count[e] = 0;
-    s_fill[e] = 0;
-  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < kAlignWarps * kMaxExperts; i += blockDim.x)
+    s_next[i / kMaxExperts][i % kMaxExperts] = 0;
+  if (threadIdx.x == 0)
+    s_max = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = topk_ids[i] - expert_start;
-    if (e >= 0 && e < num_local_experts)
-      atomicAdd(&s_count[e], 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int pos = 0;
-    for (int e = 0; e < num_local_experts; ++e) {
-      s_start[e] = pos;
-      pos += (s_count[e] + kGemmBM - 1) / kGemmBM * kGemmBM;
+  const int per_warp = ((pairs + kAlignWarps - 1) / kAlignWarps + 31) & ~31;
+  const int p0 = warp * per_warp, p1 = min(pairs, p0 + per_warp);
+  for (int base = p0; base < p1; base += 32 * kAlignBatch) {
+    int e[kAlignBatch];
+#pragma unroll
+    for (int j = 0; j < kAlignBatch; ++j) {
+      const int i = base + j * 32 + lane;
+      e[j] = i < p1 ? topk_ids[i] - expert_start : -1;
+      if (e[j] >= num_local_experts)
+        e[j] = -1;
     }
-    s_start[num_local_experts] = pos;
-    *m_total = pos < capacity ? pos : capacity;
+#pragma unroll
+    for (int j = 0; j < kAlignBatch; ++j) {
+      const unsigned same = __match_any_sync(0xffffffffu, e[j]);
+      if (e[j] >= 0 && lane == __ffs(same) - 1)
+        s_next[warp][e[j]] += __popc(same);
+      __syncwarp();
+    }
   }
   __syncthreads();
-  const int total = min(s_start[num_local_experts], capacity);
-  for (int i = threadIdx.x; i < total; i += blockDim.x) {
-    a_idx[i] = -1;
-    pair_idx[i] = -1;
-    pair_w[i] = 0.f;
+  // positions: experts in order, warps in order inside an expert
+  int count = 0, tiles = 0;
+  if (threadIdx.x < kMaxExperts) {
+    const int e = threadIdx.x;
+    for (int w = 0; w < kAlignWarps; ++w) {
+      const int c = s_next[w][e];
+      s_next[w][e] = count;
+      count += c;
+    }
+    const int even = (count + kPgMaxRows - 1) / kPgMaxRows;
+    const int h = count ? ((count + even - 1) / even + 31) & ~31 : 32;
+    tiles = (count + h - 1) / h;
+    int c_incl = count, t_incl = tiles;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int oc = __shfl_up_sync(0xffffffffu, c_incl, off), ot = __shfl_up_sync(0xffffffffu, t_incl, off);
+      if (lane >= off) {
+        c_incl += oc;
+        t_incl += ot;
+      }
+    }
+    if (lane == 31) {
+      s_warp[0][warp] = c_incl;
+      s_warp[1][warp] = t_incl;
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    int c_first = c_incl - count, t_first = t_incl - tiles;
+    for (int w = 0; w < warp; ++w) {
+      c_first += s_warp[0][w];
+      t_first += s_warp[1][w];
+    }
+    for (int w = 0; w < kAlignWarps; ++w)
+      s_next[w][e] += c_first;
+    if (tiles > 0) {
+      for (int t = 0; t < tiles; ++t)
+        row_tiles[t_first + t] = make_int4(c_first + t * h, min(h, count - t * h), e, 0);
+      atomicMax(&s_max, min(h, count));
+    }
+    if (e == kMaxExperts - 1)
+      tiles_dev[0] = t_first + tiles;
   }
-  for (int e = threadIdx.x; e < num_local_experts; e += blockDim.x)
-    for (int t = s_start[e] / kGemmBM; t < s_start[e + 1] / kGemmBM; ++t)
-      tile_expert[t] = e;
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = topk_ids[i] - expert_start;
-    if (e < 0 || e >= num_local_experts)
-      continue;
-    const int pos = s_start[e] + atomicAdd(&s_fill[e], 1);
-    if (pos >= capacity)
-      continue;
-    const int row = i / top_k;
-    a_idx[pos] = row_src ? row_src[row] : row;
-    pair_idx[pos] = i;
-    pair_w[pos] = topk_w[i];
+  if (threadIdx.x == 0)
+    tiles_dev[1] = s_max;
+  for (int base = p0; base < p1; base += 32 * kAlignBatch) {
+    int e[kAlignBatch];
+#pragma unroll
+    for (int j = 0; j < kAlignBatch; ++j) {
+      const int i = base + j * 32 + lane;
+      e[j] = i < p1 ? topk_ids[i] - expert_start : -1;
+      if (e[j] >= num_local_experts)
+        e[j] = -1;
+    }
+#pragma unroll
+    for (int j = 0; j < kAlignBatch; ++j) {
+      const int i = base + j * 32 + lane;
+      const unsigned same = __match_any_sync(0xffffffffu, e[j]);
+      int pos = -1;
+      if (e[j] >= 0)
+        pos = s_next[warp][e[j]] + __popc(same & ((1u << lane) - 1u));
+      if (i < p1)
+        pair_pos[i] = pos;
+      __syncwarp();
+      if (e[j] >= 0 && lane == __ffs(same) - 1)
+        s_next[warp][e[j]] += __popc(same);
+      __syncwarp();
+    }
+  }
+}
+
+// staged[pos] = x row of every owned pair, pair_idx[pos] = pair, pair_w[pos] = its routing weight: one warp per row of x,
+// which it reads once and writes to the row's top_k positions.
+__global__ void __launch_bounds__(256)
+moe_stage_kernel(const uint4* __restrict__ x, int64_t x_pitch_vecs, const int32_t* __restrict__ idx, int x_rows,
+                 const int32_t* __restrict__ pair_pos, const float* __restrict__ topk_w, int num_rows,
+                 const int32_t* __restrict__ num_rows_dev, int top_k, uint4* __restrict__ staged, int vecs,
+                 int32_t* __restrict__ pair_idx, float* __restrict__ pair_w) {
+  pdl_wait();      // programmatic dependent launch: nothing before this reads an earlier kernel's data
+  pdl_trigger();
+  const int n = num_rows_dev ? min(num_rows, *num_rows_dev) : num_rows;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int m = blockIdx.x * 8 + warp; m < n; m += gridDim.x * 8) {
+    const int r = idx ? min(max(idx[m], 0), x_rows - 1) : m;
+    const uint4* src = x + static_cast<int64_t>(r) * x_pitch_vecs;
+    const int my_pos = lane < top_k ? pair_pos[static_cast<int64_t>(m) * top_k + lane] : -1;   // top_k <= 16
+    if (my_pos >= 0) {
+      const int i = m * top_k + lane;
+      pair_idx[my_pos] = i;
+      pair_w[my_pos] = topk_w[i];
+    }
+    for (int base = 0; base < vecs; base += 128) {   // uniform over the warp
+      const int v0 = base + lane;
+      uint4 a[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (v0 + j * 32 < vecs)
+          a[j] = __ldg(src + v0 + j * 32);
+      for (int k = 0; k < top_k; ++k) {
+        const int pos = __shfl_sync(0xffffffffu, my_pos, k);
+        if (pos < 0)
+          continue;
+        uint4* dst = staged + static_cast<int64_t>(pos) * vecs;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (v0 + j * 32 < vecs)
+            dst[v0 + j * 32] = a[j];
+      }
+    }
   }
 }
 
@@ -215,23 +308,22 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restric
 size_t align_up_sz(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct MoeLayout {
-  int capacity;        // padded (row, slot) positions
-  size_t off_a_idx, off_pair_idx, off_pair_w, off_tile_expert, off_m_total, off_staged, off_inter, off_y, total;
+  int pairs;           // (row, slot) positions
+  size_t off_pos, off_pair_idx, off_pair_w, off_tiles, off_counts, off_staged, off_inter, off_y, total;
 };
 
 MoeLayout moe_layout(int max_rows, int top_k, int num_local_experts, int hidden, int inter) {
   MoeLayout l;
   const int64_t pairs = static_cast<int64_t>(max_rows) * top_k;
-  const int64_t cap = (pairs + static_cast<int64_t>(num_local_experts) * (kGemmBM - 1) + kGemmBM - 1) / kGemmBM * kGemmBM;
-  l.capacity = static_cast<int>(cap);
+  l.pairs = static_cast<int>(pairs);
   size_t off = 0;
-  l.off_a_idx = off;       off = align_up_sz(off + cap * 4, 1024);
-  l.off_pair_idx = off;    off = align_up_sz(off + cap * 4, 1024);
-  l.off_pair_w = off;      off = align_up_sz(off + cap * 4, 1024);
-  l.off_tile_expert = off; off = align_up_sz(off + (cap / kGemmBM) * 4, 1024);
-  l.off_m_total = off;     off = align_up_sz(off + 16, 1024);
-  l.off_staged = off;      off = align_up_sz(off + cap * static_cast<size_t>(hidden) * 2, 1024);
-  l.off_inter = off;       off = align_up_sz(off + cap * static_cast<size_t>(inter) * 2, 1024);
+  l.off_pos = off;         off = align_up_sz(off + pairs * 4, 1024);
+  l.off_pair_idx = off;    off = align_up_sz(off + pairs * 4, 1024);
+  l.off_pair_w = off;      off = align_up_sz(off + pairs * 4, 1024);
+  l.off_tiles = off;       off = align_up_sz(off + (pairs / kPgMaxRows + num_local_experts) * sizeof(int4), 1024);
+  l.off_counts = off;      off = align_up_sz(off + 16, 1024);
+  l.off_staged = off;      off = align_up_sz(off + static_cast<size_t>(pairs) * hidden * 2, 1024);
+  l.off_inter = off;       off = align_up_sz(off + static_cast<size_t>(pairs) * inter * 2, 1024);
   l.off_y = off;           off = align_up_sz(off + static_cast<size_t>(pairs) * hidden * 2, 1024);
   l.total = off;
   return l;
@@ -290,57 +382,48 @@ int dyllm_moe_ffn(const void* x, int x_rows, int hidden, int64_t ldx, const int3
                 "moe_ffn: needs a 16-byte aligned workspace of %zu bytes (got %zu)", l.total, workspace_bytes);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  int32_t* a_idx = reinterpret_cast<int32_t*>(ws + l.off_a_idx);
+  int32_t* pair_pos = reinterpret_cast<int32_t*>(ws + l.off_pos);
   int32_t* pair_idx = reinterpret_cast<int32_t*>(ws + l.off_pair_idx);
   float* pair_w = reinterpret_cast<float*>(ws + l.off_pair_w);
-  int32_t* tile_expert = reinterpret_cast<int32_t*>(ws + l.off_tile_expert);
-  int32_t* m_total = reinterpret_cast<int32_t*>(ws + l.off_m_total);
+  int4* row_tiles = reinterpret_cast<int4*>(ws + l.off_tiles);
+  int32_t* tiles_dev = reinterpret_cast<int32_t*>(ws + l.off_counts);
   void* staged = ws + l.off_staged;
   __nv_bfloat16* inter_buf = reinterpret_cast<__nv_bfloat16*>(ws + l.off_inter);
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(ws + l.off_y);
 
-  DYLLM_LAUNCH(moe_align_kernel, 1, 1024, 0, s, topk_ids, topk_weights, num_rows, num_rows_dev, top_k, expert_start,
-                                      num_local_experts, idx, a_idx, pair_idx, pair_w, tile_expert, m_total, l.capacity);
+  DYLLM_LAUNCH(moe_align_kernel, 1, kAlignWarps * 32, 0, s, topk_ids, num_rows, num_rows_dev, top_k, expert_start,
+               num_local_experts, pair_pos, row_tiles, tiles_dev);
   int rc = check_launch("moe_align");
   if (rc != DYLLM_OK)
     return rc;
   const int hint_rows = rows_hint > 0 && rows_hint < num_rows ? rows_hint : num_rows;
-  int64_t hint64 = static_cast<int64_t>(hint_rows) * top_k + static_cast<int64_t>(num_local_experts) * (kGemmBM / 2);
-  const int hint = hint64 < l.capacity ? static_cast<int>(hint64) : l.capacity;
-
-  // rows of x for every padded position (padding reads row 0), then plain TMA boxes
-  rc = stage_rows(x, ldx, a_idx, x_rows, staged, hidden, l.capacity, m_total, hint, s);
+  DYLLM_LAUNCH(moe_stage_kernel, min(cdiv_i(hint_rows, 8), sm_count() * 8), 256, 0, s, static_cast<const uint4*>(x),
+               ldx / 8, idx, x_rows, pair_pos, topk_weights, num_rows, num_rows_dev, top_k,
+               static_cast<uint4*>(staged), hidden / 8, pair_idx, pair_w);
+  rc = check_launch("moe_stage");
   if (rc != DYLLM_OK)
     return rc;
-  GemmParams g1 = {};
-  g1.a = static_cast<const __nv_bfloat16*>(staged);
-  g1.a_rows = l.capacity;
-  g1.m_count_dev = m_total;
-  g1.tile_expert = tile_expert;
-  g1.M = l.capacity;
-  g1.K = hidden;
-  g1.b_rows_per_expert = 2 * inter;
-  g1.up_row_offset = inter;
-  g1.out = inter_buf;
-  g1.ldc = inter;
-  rc = launch_gathered_gemm(true, 0, 0, g1, hidden, w1, static_cast<int64_t>(num_local_experts) * 2 * inter, inter, hint,
-                            nullptr, s);
+  PairGemmParams g = {};
+  g.row_tiles = row_tiles;
+  g.tiles_dev = tiles_dev;
+  g.K = hidden;
+  g.n = inter;
+  g.w_rows_per_block = 2 * inter;
+  g.up_row_offset = inter;
+  g.out = inter_buf;
+  g.ldc = inter;
+  rc = launch_pair_gemm(true, g, staged, l.pairs, hidden, w1, static_cast<int64_t>(num_local_experts) * 2 * inter, s);
   if (rc != DYLLM_OK)
     return rc;
-  GemmParams g2 = {};
-  g2.a = inter_buf;
-  g2.a_rows = l.capacity;
-  g2.m_count_dev = m_total;
-  g2.tile_expert = tile_expert;
-  g2.M = l.capacity;
-  g2.K = inter;
-  g2.b_rows_per_expert = hidden;
-  g2.out = y;
-  g2.ldc = hidden;
-  g2.out_row_map = pair_idx;
-  g2.row_scale = pair_w;
-  rc = launch_gathered_gemm(false, 0, 0, g2, inter, w2, static_cast<int64_t>(num_local_experts) * hidden, hidden, hint,
-                            nullptr, s);
+  g.K = inter;
+  g.n = hidden;
+  g.w_rows_per_block = hidden;
+  g.up_row_offset = 0;
+  g.out = y;
+  g.ldc = hidden;
+  g.out_row_map = pair_idx;
+  g.row_scale = pair_w;
+  rc = launch_pair_gemm(false, g, inter_buf, l.pairs, inter, w2, static_cast<int64_t>(num_local_experts) * hidden, s);
   if (rc != DYLLM_OK)
     return rc;
   const int blocks = min(hint_rows, sm_count() * 8);

@@ -1,0 +1,93 @@
+// Launch of the CTA-pair GEMM (pair_gemm.cuh).
+#include <atomic>
+
+#include "pair_gemm.cuh"
+
+namespace dyllm {
+
+namespace {
+
+// Arrival counters of the tiles that are cut along k: zero between launches (the last arrival resets its counter).  Calls
+// that may run at the same time have different workspaces, so the workspace picks the set of counters; two workspaces
+// share a set with a probability of 1 / 256.
+constexpr int kPgTicketSets = 256;
+constexpr int kPgTickets = 384;                  // two per cut tile, of which there are at most an eighth of the CTA slots
+__device__ int g_pair_tickets[kPgTicketSets * kPgTickets] = {0};
+std::atomic<int*> g_pair_tickets_ptr[64];
+
+int* pair_tickets(const void* workspace) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+    return nullptr;
+  int* base = g_pair_tickets_ptr[dev].load(std::memory_order_acquire);
+  if (!base) {
+    void* sym = nullptr;
+    if (cudaGetSymbolAddress(&sym, g_pair_tickets) != cudaSuccess)
+      return nullptr;
+    base = static_cast<int*>(sym);
+    g_pair_tickets_ptr[dev].store(base, std::memory_order_release);   // every thread finds the same address
+  }
+  const uint64_t h = (reinterpret_cast<uintptr_t>(workspace) >> 8) * 0x9E3779B97F4A7C15ull;
+  return base + (h >> 56) * kPgTickets;
+}
+
+template <bool SWIGLU>
+int launch(const CUtensorMap (&t)[5], const PairGemmParams& p, int pairs, cudaStream_t stream) {
+  auto kernel = pair_gemm_kernel<SWIGLU>;
+  // one flag per kernel instantiation and device: the opt-in shared-memory size is a per-function attribute
+  static std::atomic<bool> smem_set[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  dev = (dev < 0 || dev >= 64) ? 0 : dev;
+  if (!smem_set[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPgSmem)) != cudaSuccess)
+      return set_error(DYLLM_ERR_CUDA, "cudaFuncSetAttribute(%u bytes of shared memory) failed: %s", kPgSmem,
+                       cudaGetErrorString(cudaGetLastError()));
+    smem_set[dev].store(true, std::memory_order_release);
+  }
+  launch_pdl_cluster(kernel, dim3(2 * pairs), dim3(kPgThreads), kPgSmem, stream, 2, t[0], t[1], t[2], t[3], t[4], p);
+  return check_launch("pair_gemm");
+}
+
+}  // namespace
+
+// `a` holds a_rows rows of pitch lda (p.M dense rows, or the rows that p.row_tiles list); `w` holds w_total_rows rows
+// of p.K.  p.status_word and p.tickets are filled in here.
+int launch_pair_gemm(bool swiglu, const PairGemmParams& p_in, const void* a, int a_rows, int64_t lda, const void* w,
+                     int64_t w_total_rows, cudaStream_t stream) {
+  PairGemmParams p = p_in;
+  DYLLM_REQUIRE(p.K > 0 && p.K % 64 == 0, DYLLM_ERR_UNSUPPORTED, "gemm: K = %d is not a multiple of 64", p.K);
+  DYLLM_REQUIRE(p.n > 0 && p.n % 64 == 0, DYLLM_ERR_UNSUPPORTED, "gemm: N = %d is not a multiple of 64", p.n);
+  DYLLM_REQUIRE(lda % 8 == 0 && p.ldc % 8 == 0 && p.ldc2 % 8 == 0, DYLLM_ERR_UNSUPPORTED,
+                "gemm: row pitches must be multiples of 8");
+  DYLLM_REQUIRE((reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
+                    (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.out2) & 15) == 0,
+                DYLLM_ERR_INVALID_ARGUMENT, "gemm: operands must be 16-byte aligned");
+  DYLLM_REQUIRE(!p.out2 || (p.split_col > 0 && p.split_col % 128 == 0 && p.split_col < p.n), DYLLM_ERR_INVALID_ARGUMENT,
+                "gemm: split column %d must be a multiple of 128 inside (0, %d)", p.split_col, p.n);
+  if (p.M <= 0 && !p.row_tiles)
+    return DYLLM_OK;
+  int pairs = sm_count() / 2;
+  pairs = pairs < 1 ? 1 : (pairs > kPgMaxPairs ? kPgMaxPairs : pairs);
+  p.status_word = device_status_word();
+  p.tickets = p.partial ? pair_tickets(p.partial) : nullptr;
+  p.split_slots = 2 * sm_count();
+  if (!p.tickets)
+    p.partial = nullptr;
+  // boxes of one k step (64 columns) and, as 3-D boxes [k step][row][column], of two
+  CUtensorMap t[5];
+  int rc = encode_tmap_2d_bf16(&t[0], w, w_total_rows, p.K, p.K, 128, 64, true);
+  if (rc == DYLLM_OK)
+    rc = encode_tmap_2d_bf16(&t[1], a, a_rows, p.K, lda, 32, 64, true);
+  if (rc == DYLLM_OK)
+    rc = encode_tmap_3d_bf16(&t[2], w, 64, w_total_rows, p.K / 64, static_cast<uint64_t>(p.K) * 2, 128, 64, 128, 2, true);
+  if (rc == DYLLM_OK)
+    rc = encode_tmap_3d_bf16(&t[3], a, 64, a_rows, p.K / 64, static_cast<uint64_t>(lda) * 2, 128, 64, 32, 2, true);
+  if (rc == DYLLM_OK)
+    rc = encode_tmap_3d_bf16(&t[4], a, 64, a_rows, p.K / 64, static_cast<uint64_t>(lda) * 2, 128, 64, 64, 2, true);
+  if (rc != DYLLM_OK)
+    return rc;
+  return swiglu ? launch<true>(t, p, pairs, stream) : launch<false>(t, p, pairs, stream);
+}
+
+}  // namespace dyllm

@@ -250,7 +250,7 @@ class ColumnParallelLinear(LinearBase):
         return _project(x, self.weight, self.bias)
 
     def forward_gathered(self, x: torch.Tensor, idx32: torch.Tensor | None, num_rows: int, num_rows_dev=None,
-                         rows_hint: int = 0, split_col: int = 0, out=None):
+                         rows_hint: int = 0, split_col: int = 0, out=None, few_rows_ctas: int = 0):
         """``self(x[idx])`` on the tcgen05 GEMM; ``num_rows`` may be a capacity with the live count on the
         device.  ``idx32`` None: ``x`` already holds the rows packed in list order.  With ``split_col`` the
         output columns are returned as two tensors (K and V halves); ``out`` may bring them (a pair)."""
@@ -263,7 +263,7 @@ class ColumnParallelLinear(LinearBase):
         else:
             out, out2 = torch.empty((num_rows, n_out), dtype=x.dtype, device=x.device), None
         ops.gathered_linear(x, self.weight, idx32, num_rows=num_rows, num_rows_dev=num_rows_dev, rows_hint=rows_hint,
-                            out=out, out2=out2, split_col=split_col)
+                            out=out, out2=out2, split_col=split_col, few_rows_ctas=few_rows_ctas)
         if self.bias is not None:
             out += self.bias[: out.size(1)]
             if out2 is not None:

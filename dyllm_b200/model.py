@@ -148,9 +148,17 @@ def _forward_sparse_overlapped(self, positions, hidden_states, salient_rows):
     v_new = torch.empty((cap, self.kv_size), dtype=hidden_states.dtype, device=dev)
     dv = torch.empty((cap, Hkv, D), dtype=hidden_states.dtype, device=dev)
     rows_k = ctx.idx_salient_row_k if ctx.idx_salient_row_k is not None else ctx.idx_salient_row
-    side.wait_stream(main)
+    # The query projection is launched first: it fills the SMs, and what its last wave leaves idle is where the other
+    # branch belongs.  (The other way round that branch takes SMs from the first wave, which then needs one wave more.)
+    forked = main.record_event()
+    q = self.q_proj(hidden_states).view(-1, H, D)
+    side.wait_event(forked)
+    # Beside a query projection of many rows the few salient rows' product keeps to 40 SMs, about what the library
+    # kernel's last wave leaves idle: the weights stream in under it either way.  A short one has no such tail.
+    ctas = 40 if hidden_states.size(0) >= 2048 else 0
     with torch.cuda.stream(side):
-        self.kv_proj.forward_gathered(salient_rows, None, cap, n_dev, hint, split_col=self.kv_size, out=(k_new, v_new))
+        self.kv_proj.forward_gathered(salient_rows, None, cap, n_dev, hint, split_col=self.kv_size, out=(k_new, v_new),
+                                      few_rows_ctas=ctas)
         k3 = k_new.view(cap, Hkv, D)
         if self.k_norm is not None:
             k3 = self.k_norm.forward_heads_(k3, n_dev)
@@ -158,7 +166,6 @@ def _forward_sparse_overlapped(self, positions, hidden_states, salient_rows):
                             self.rotary_emb.cos_sin_cache.view(-1, D), ctx.cu_seqlens_k, self.k_cache.seq_start_gpu,
                             self.attn.v_cache.seq_start_gpu, md.running_seqs_tensor, self.k_cache.cache,
                             self.attn.v_cache.cache, n_dev, dv=dv)
-    q = self.q_proj(hidden_states).view(-1, H, D)
     if self.q_norm is not None:
         q = self.q_norm.forward_heads_(q)
     q = self.rotary_emb.rotate(positions, q)

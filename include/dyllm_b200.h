@@ -159,10 +159,10 @@ size_t dyllm_gathered_linear_workspace_bytes(int max_rows, int in_features, int 
  * out_row_map null = m (negative entries drop the row), row_scale null = 1.  When out2 is not null,
  * output columns >= split_col (a multiple of 128) go to out2[.., column - split_col] instead (used to
  * write K and V of the fused K/V projection into two tensors).  in_features % 64 == 0,
- * out_features % 64 == 0.  Few rows and few column tiles switch on a deterministic split-K: the k range is
- * cut into at most 4 parts whose fp32 partial sums go to the workspace, and the CTA that finishes an output
- * tile last adds them in split order inside the same launch (arrival counters live in a small array inside
- * the library, so two split-K calls on one device must not overlap on the GPU: issue them on one stream).
+ * out_features % 64 == 0.  Tiles that would leave many SMs idle are cut along k (deterministic: fp32 partial sums go to
+ * the workspace, and the CTA that finishes an output tile last adds them in k order inside the same launch).  Arrival
+ * counters live in a small array inside the library, chosen by the workspace: calls that share a workspace must not
+ * overlap on the GPU (issue them on one stream), nor calls that name a tile width or a_mode 1.
  * ref: dyllm/model_executor/models/llada.py:108 (kv_proj(hidden_states[idx_salient_row])),
  *      dyllm/model_executor/layers/linear.py:50-51. */
 int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ldx, const int32_t* idx,
@@ -170,6 +170,17 @@ int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ld
                           int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
                           const int32_t* out_row_map, const float* row_scale, void* workspace,
                           size_t workspace_bytes, int a_mode, int tile_n, void* stream);
+/* The same call with two more arguments.  bias (bf16 [out_features], nullable) is added to the bf16 result (a second
+ * rounding, as a separate addition has it); only with a_mode <= 0 and tile_n 0.  few_rows_ctas serves a stream that runs beside another one: while all live rows fit one row tile (256 rows) the
+ * product keeps to `few_rows_ctas` CTAs (one per SM; 0 = all SMs), so that a kernel on the other stream finds the
+ * remaining SMs free.  Ignored by calls that name a tile width or a_mode 1. */
+int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64_t ldx, const int32_t* idx,
+                               int num_rows, const int32_t* num_rows_dev, int rows_hint, const void* weight,
+                                 int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
+                                 const int32_t* out_row_map, const float* row_scale, void* workspace,
+                                 size_t workspace_bytes, int a_mode, int tile_n, const void* bias, int few_rows_ctas,
+                                 void* stream);
+
 
 /* Bytes of workspace dyllm_swiglu_ffn needs for up to max_rows gathered rows. */
 size_t dyllm_swiglu_ffn_workspace_bytes(int max_rows, int hidden, int inter);
