@@ -189,10 +189,7 @@ def set_projection_backend(name: str) -> None:
 
 def _project(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None) -> torch.Tensor:
     if _projection_backend == "tcgen05" and x.is_cuda and x.dim() == 2 and x.size(0) > 0:
-        y = ops.gathered_linear(x.contiguous(), weight, None, num_rows=x.size(0), rows_hint=x.size(0))
-        if bias is not None:
-            y += bias
-        return y
+        return ops.gathered_linear(x.contiguous(), weight, None, num_rows=x.size(0), rows_hint=x.size(0), bias=bias)
     return F.linear(x, weight, bias)
 
 
@@ -263,11 +260,7 @@ class ColumnParallelLinear(LinearBase):
         else:
             out, out2 = torch.empty((num_rows, n_out), dtype=x.dtype, device=x.device), None
         ops.gathered_linear(x, self.weight, idx32, num_rows=num_rows, num_rows_dev=num_rows_dev, rows_hint=rows_hint,
-                            out=out, out2=out2, split_col=split_col, few_rows_ctas=few_rows_ctas)
-        if self.bias is not None:
-            out += self.bias[: out.size(1)]
-            if out2 is not None:
-                out2 += self.bias[out.size(1):]
+                            out=out, out2=out2, split_col=split_col, few_rows_ctas=few_rows_ctas, bias=self.bias)
         return (out, out2) if split_col else out
 
 
