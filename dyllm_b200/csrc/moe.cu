@@ -17,43 +17,87 @@ namespace {
 constexpr int kMaxExperts = 256;
 constexpr int kMaxTopK = 16;
 
-// One block (256 threads) per row: 8 warps split the experts, lanes split the hidden dimension.
-__global__ void __launch_bounds__(256)
-moe_route_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __restrict__ idx, int x_rows,
-                 int num_rows, const int32_t* __restrict__ num_rows_dev, const __nv_bfloat16* __restrict__ wr,
-                 int hidden, int num_experts, int top_k, int renormalize, float* __restrict__ topk_w,
-                 int32_t* __restrict__ topk_ids) {
-  pdl_wait();      // programmatic dependent launch: nothing before this reads an earlier kernel's data
-  pdl_trigger();
-  const int n = num_rows_dev ? min(num_rows, *num_rows_dev) : num_rows;
-  __shared__ float s_logits[kMaxExperts];
+// Router.  A block takes R rows at a time, its 16 warps share out the experts in pairs, lanes split the hidden
+// dimension.  Several rows wait in shared memory, so a weight vector fetched from L2 serves R rows: with one row per block
+// 3003 rows read the 256 KB router weight (64 experts, hidden 2048) 3003 times, 88 us.  Few rows are bound by the latency
+// of the weight loads instead: R = 1 spreads them over more blocks, and a lane keeps eight loads in flight (150 rows:
+// 21 us with one expert and one load at a time).
+constexpr int kRouteThreads = 512;
+constexpr int kRouteManyRows = 4;
+
+template <int R>
+__device__ __forceinline__ void
+route_rows(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __restrict__ idx, int x_rows, int n,
+           const __nv_bfloat16* __restrict__ wr, int hidden, int num_experts, int top_k, int renormalize,
+           float* __restrict__ topk_w, int32_t* __restrict__ topk_ids, uint4* s_x, float (*s_all)[kMaxExperts]) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int m = blockIdx.x; m < n; m += gridDim.x) {
-    const int r = idx ? min(max(idx[m], 0), x_rows - 1) : m;
-    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(r) * ldx);
-    const int vecs = hidden / 8;
-    for (int e = warp; e < num_experts; e += 8) {
-      const uint4* w = reinterpret_cast<const uint4*>(wr + static_cast<int64_t>(e) * hidden);
-      float acc = 0.f;
-      for (int v = lane; v < vecs; v += 32) {
-        const uint4 a = __ldg(xr + v), b = __ldg(w + v);
-        const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
-        const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
+  const int vecs = hidden / 8;
+  for (int m0 = blockIdx.x * R; m0 < n; m0 += gridDim.x * R) {
+    const uint4* xr = nullptr;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int m = min(m0 + j, n - 1);
+      const int r = idx ? min(max(idx[m], 0), x_rows - 1) : m;
+      xr = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(r) * ldx);
+      if (R > 1)
+        for (int v = threadIdx.x; v < vecs; v += kRouteThreads)
+          s_x[j * vecs + v] = __ldg(xr + v);
+    }
+    if (R > 1)
+      __syncthreads();
+    for (int e = warp * 2; e < num_experts; e += kRouteThreads / 16) {
+      const bool two = e + 1 < num_experts;
+      const uint4* w0 = reinterpret_cast<const uint4*>(wr + static_cast<int64_t>(e) * hidden);
+      const uint4* w1 = two ? w0 + vecs : w0;
+      float acc[2][R];
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        acc[0][j] = acc[1][j] = 0.f;
+      for (int v0 = lane; v0 < vecs; v0 += 128) {
+        uint4 w[2][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float2 fa = __bfloat1622float2(a2[i]), fb = __bfloat1622float2(b2[i]);
-          acc = fmaf(fa.x, fb.x, acc);
-          acc = fmaf(fa.y, fb.y, acc);
+          const int v = v0 + i * 32;
+          w[0][i] = v < vecs ? __ldg(w0 + v) : make_uint4(0, 0, 0, 0);
+          w[1][i] = v < vecs ? __ldg(w1 + v) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int v = v0 + i * 32;
+          if (v >= vecs)
+            break;
+#pragma unroll
+          for (int j = 0; j < R; ++j) {
+            const uint4 a = R > 1 ? s_x[j * vecs + v] : __ldg(xr + v);
+            const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+              const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&w[z][i]);
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const float2 fa = __bfloat1622float2(a2[c]), fb = __bfloat1622float2(b2[c]);
+                acc[z][j] = fmaf(fa.x, fb.x, acc[z][j]);
+                acc[z][j] = fmaf(fa.y, fb.y, acc[z][j]);
+              }
+            }
+          }
         }
       }
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-        acc += __shfl_xor_sync(0xffffffffu, acc, off);
-      if (lane == 0)
-        s_logits[e] = acc;
+      for (int z = 0; z < 2; ++z)
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1)
+            acc[z][j] += __shfl_xor_sync(0xffffffffu, acc[z][j], off);
+          if (lane == 0 && (z == 0 || two))
+            s_all[j][e + z] = acc[z][j];
+        }
     }
     __syncthreads();
-    if (warp == 0) {
+    const int m = m0 + warp;
+    if (warp < R && m < n) {
+      float* s_logits = s_all[warp];
       // softmax over the experts, then top-k by repeated arg-max (lowest index wins ties)
       float mx = -3.0e38f;
       for (int e = lane; e < num_experts; e += 32)
@@ -111,6 +155,24 @@ moe_route_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t
     }
     __syncthreads();
   }
+}
+
+// `shared_rows`: rows that the dynamic shared memory holds (0: always one row per block at a time).
+__global__ void __launch_bounds__(kRouteThreads, 2)
+moe_route_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __restrict__ idx, int x_rows,
+                 int num_rows, const int32_t* __restrict__ num_rows_dev, const __nv_bfloat16* __restrict__ wr,
+                 int hidden, int num_experts, int top_k, int renormalize, float* __restrict__ topk_w,
+                 int32_t* __restrict__ topk_ids, int shared_rows) {
+  pdl_wait();      // programmatic dependent launch: nothing before this reads an earlier kernel's data
+  pdl_trigger();
+  extern __shared__ uint4 s_x[];                 // [kRouteManyRows][hidden / 8]
+  __shared__ float s_all[kRouteManyRows][kMaxExperts];
+  const int n = num_rows_dev ? min(num_rows, *num_rows_dev) : num_rows;
+  // several rows per block once there are enough rows for more than one turn of the grid
+  if (shared_rows >= kRouteManyRows && n > static_cast<int>(gridDim.x))
+    route_rows<kRouteManyRows>(x, ldx, idx, x_rows, n, wr, hidden, num_experts, top_k, renormalize, topk_w, topk_ids, s_x, s_all);
+  else
+    route_rows<1>(x, ldx, idx, x_rows, n, wr, hidden, num_experts, top_k, renormalize, topk_w, topk_ids, s_x, s_all);
 }
 
 // Single block: the position of every owned (row, slot) pair when the pairs are grouped by local expert, in pair order
@@ -348,10 +410,14 @@ int dyllm_moe_route(const void* x, int x_rows, int hidden, int64_t ldx, const in
   if (num_rows == 0 || x_rows == 0)
     return DYLLM_OK;
   DYLLM_REQUIRE(x && router_weight && topk_weights && topk_ids, DYLLM_ERR_INVALID_ARGUMENT, "moe_route: null pointer");
-  const int blocks = min(num_rows, sm_count() * 8);
-  DYLLM_LAUNCH(moe_route_kernel, blocks, 256, 0, static_cast<cudaStream_t>(stream), 
+  // the live count is known on the device only: the kernel chooses between one and several rows per block
+  const int shared_rows = num_rows >= kRouteManyRows && kRouteManyRows * hidden * 2 <= 40 * 1024 ? kRouteManyRows : 0;
+  const int blocks = min(num_rows, 2 * sm_count());
+  DYLLM_LAUNCH(moe_route_kernel, blocks, kRouteThreads, static_cast<size_t>(shared_rows) * hidden * 2,
+      static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(x), ldx, idx, x_rows, num_rows, num_rows_dev,
-      static_cast<const __nv_bfloat16*>(router_weight), hidden, num_experts, top_k, renormalize, topk_weights, topk_ids);
+      static_cast<const __nv_bfloat16*>(router_weight), hidden, num_experts, top_k, renormalize, topk_weights, topk_ids,
+      shared_rows);
   return check_launch("moe_route");
 }
 
