@@ -131,7 +131,7 @@ bool few_tiles(bool swiglu, int n, int K, int num_rows, const int32_t* num_rows_
   if (h > kSplitRows)
     return false;
   if (swiglu)
-    return n < 6144 || (!num_rows_dev && num_rows > 64 && num_rows <= 128);
+    return !num_rows_dev && num_rows > 64 && num_rows <= 128;
   return n <= 2048 || K < 2048;
 }
 

@@ -45,8 +45,9 @@ route_rows(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __re
     }
     if (R > 1)
       __syncthreads();
-    for (int e = warp * 2; e < num_experts; e += kRouteThreads / 16) {
-      const bool two = e + 1 < num_experts;
+    const int per_warp = num_experts > kRouteThreads / 32 ? 2 : 1;
+    for (int e = warp * per_warp; e < num_experts; e += kRouteThreads / 32 * per_warp) {
+      const bool two = per_warp == 2 && e + 1 < num_experts;
       const uint4* w0 = reinterpret_cast<const uint4*>(wr + static_cast<int64_t>(e) * hidden);
       const uint4* w1 = two ? w0 + vecs : w0;
       float acc[2][R];

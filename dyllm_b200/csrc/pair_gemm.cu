@@ -32,7 +32,7 @@ int* pair_tickets(const void* workspace) {
 }
 
 template <bool SWIGLU>
-int launch(const CUtensorMap (&t)[5], const PairGemmParams& p, int pairs, cudaStream_t stream) {
+int launch(const CUtensorMap (&t)[6], const PairGemmParams& p, int pairs, cudaStream_t stream) {
   auto kernel = pair_gemm_kernel<SWIGLU>;
   // one flag per kernel instantiation and device: the opt-in shared-memory size is a per-function attribute
   static std::atomic<bool> smem_set[64];
@@ -45,7 +45,7 @@ int launch(const CUtensorMap (&t)[5], const PairGemmParams& p, int pairs, cudaSt
                        cudaGetErrorString(cudaGetLastError()));
     smem_set[dev].store(true, std::memory_order_release);
   }
-  launch_pdl_cluster(kernel, dim3(2 * pairs), dim3(kPgThreads), kPgSmem, stream, 2, t[0], t[1], t[2], t[3], t[4], p);
+  launch_pdl_cluster(kernel, dim3(2 * pairs), dim3(kPgThreads), kPgSmem, stream, 2, t[0], t[1], t[2], t[3], t[4], t[5], p);
   return check_launch("pair_gemm");
 }
 
@@ -75,7 +75,7 @@ int launch_pair_gemm(bool swiglu, const PairGemmParams& p_in, const void* a, int
   if (!p.tickets)
     p.partial = nullptr;
   // boxes of one k step (64 columns) and, as 3-D boxes [k step][row][column], of two
-  CUtensorMap t[5];
+  CUtensorMap t[6];
   int rc = encode_tmap_2d_bf16(&t[0], w, w_total_rows, p.K, p.K, 128, 64, true);
   if (rc == DYLLM_OK)
     rc = encode_tmap_2d_bf16(&t[1], a, a_rows, p.K, lda, 32, 64, true);
@@ -85,6 +85,9 @@ int launch_pair_gemm(bool swiglu, const PairGemmParams& p_in, const void* a, int
     rc = encode_tmap_3d_bf16(&t[3], a, 64, a_rows, p.K / 64, static_cast<uint64_t>(lda) * 2, 128, 64, 32, 2, true);
   if (rc == DYLLM_OK)
     rc = encode_tmap_3d_bf16(&t[4], a, 64, a_rows, p.K / 64, static_cast<uint64_t>(lda) * 2, 128, 64, 64, 2, true);
+  t[5] = t[0];
+  if (rc == DYLLM_OK && swiglu)
+    rc = encode_tmap_2d_bf16(&t[5], w, w_total_rows, p.K, p.K, 64, 64, true);
   if (rc != DYLLM_OK)
     return rc;
   return swiglu ? launch<true>(t, p, pairs, stream) : launch<false>(t, p, pairs, stream);

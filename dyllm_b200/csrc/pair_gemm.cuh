@@ -79,12 +79,14 @@ constexpr int kPgMaxRows = 256;                  // rows per tile (UMMA N)
 constexpr int kPgMaxStages = 10;
 constexpr uint32_t kPgWBytes = 128 * 64 * 2;     // one weight box
 constexpr uint32_t kPgABytes = 32 * 64 * 2;      // one activation box
+constexpr uint32_t kPgSwapBytes = 2 * 32 * 64 * 4;   // narrow SwiGLU tiles: up values on their way to the gate threads
 constexpr uint32_t kPgRing = 216 * 1024;
 constexpr uint32_t kPgSmem = kPgRing + 1024;
 constexpr int kPgRowGroup = 8;                   // row tiles that share the weight tiles in flight
 
 // How a launch's tiles are shared out; the same arithmetic in every thread of the grid.
 struct PgSched {
+  bool narrow;        // SwiGLU with 64 gate and 64 up rows in the CTA's one weight block (128 columns per pair)
   int kt, nb, tile_n, row_tiles, col_tiles, parts, part_kt, units, pairs, pair, m;
 };
 
@@ -111,14 +113,17 @@ __device__ __forceinline__ bool pg_schedule(const PairGemmParams& p, bool swiglu
     return false;
   if (!p.row_tiles && s.row_tiles == 1 && p.one_tile_pairs > 0 && p.one_tile_pairs < s.pairs)
     s.pairs = p.one_tile_pairs;
+  // Few tiles leave most pairs without work.  SwiGLU tiles of half the width give twice as many (8 experts of 1024 columns
+  // with 60 rows each: 32 tiles for 74 pairs).
+  s.narrow = swiglu && 2 * s.row_tiles * ((p.n + 255) >> 8) <= s.pairs;
+  const int pair_cols = s.narrow ? 128 : 256;
   s.parts = 1;
   if (!swiglu && !p.row_tiles && p.partial && s.m <= kSplitRows)
     s.parts = effective_splits((s.m + 127) >> 7, p.n >> 6, p.split_slots, kMaxSplits, s.kt);
   s.part_kt = (s.kt + s.parts - 1) / s.parts;
-  // A plain product with few column tiles leaves most pairs without work: more and lower row tiles (the weights come from
-  // L2 the second time) give them some.
-  if (!swiglu && !p.row_tiles)
-    while (s.tile_n > 64 && 2 * s.row_tiles * ((p.n + 255) >> 8) * s.parts <= s.pairs) {
+  // More and lower row tiles (the weights come from L2 the second time) give more pairs work, too.
+  if (!p.row_tiles)
+    while (s.tile_n > 64 && 2 * s.row_tiles * ((p.n + pair_cols - 1) / pair_cols) * s.parts <= s.pairs) {
       const int more = 2 * s.row_tiles;
       s.tile_n = ((s.m + more - 1) / more + 31) & ~31;
       s.row_tiles = (s.m + s.tile_n - 1) / s.tile_n;
@@ -128,8 +133,8 @@ __device__ __forceinline__ bool pg_schedule(const PairGemmParams& p, bool swiglu
   // against 47), and half at few rows.
   const int t1 = s.row_tiles * ((p.n + 255) >> 8), t2 = s.row_tiles * ((p.n + 511) >> 9);
   const int w1 = (t1 * s.parts + s.pairs - 1) / s.pairs, w2 = (t2 * s.parts + s.pairs - 1) / s.pairs;
-  s.nb = swiglu ? 2 : (p.row_tiles ? (s.tile_n > 128 ? 2 : 1) : (w1 * 3 <= w2 * 5 ? 1 : 2));
-  const int cols = swiglu ? 256 : s.nb * 256;
+  s.nb = swiglu ? (s.narrow ? 1 : 2) : (p.row_tiles ? (s.tile_n > 128 ? 2 : 1) : (w1 * 3 <= w2 * 5 ? 1 : 2));
+  const int cols = swiglu ? pair_cols : s.nb * 256;
   s.col_tiles = (p.n + cols - 1) / cols;
   s.units = s.row_tiles * s.col_tiles * s.parts;
   return true;
@@ -254,7 +259,7 @@ template <bool SWIGLU>
 __global__ void __launch_bounds__(kPgThreads, 1)
 pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
                  const __grid_constant__ CUtensorMap tmap_w2, const __grid_constant__ CUtensorMap tmap_a2_32,
-                 const __grid_constant__ CUtensorMap tmap_a2_64,
+                 const __grid_constant__ CUtensorMap tmap_a2_64, const __grid_constant__ CUtensorMap tmap_w64,
                  const PairGemmParams p) {
   pdl_wait();      // programmatic dependent launch: nothing before this reads an earlier kernel's data
   pdl_trigger();
@@ -285,7 +290,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const CUtensorMap* const tmap_a2 = s.tile_n <= 64 ? &tmap_a2_32 : &tmap_a2_64;   // rows of the activation box
   const uint32_t a_step = ((s.tile_n + 63) >> 6) * kPgABytes;                      // activation bytes per k step
   const uint32_t stage_bytes = kps * (s.nb * kPgWBytes + a_step);
-  const int stages = min(kPgMaxStages, static_cast<int>(kPgRing / stage_bytes));
+  const int stages = min(kPgMaxStages, static_cast<int>((kPgRing - (s.narrow ? kPgSwapBytes : 0)) / stage_bytes));
   const int accs = 2 * s.nb * s.tile_n <= 512 ? 2 : 1;   // accumulators that fit the tensor memory
 
   if (threadIdx.x == 0) {
@@ -323,7 +328,9 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         const int half = t.n >> 1;
         const int boxes = (half + 31) >> 5;
         const uint32_t pair_bytes = 2 * kps * (s.nb * kPgWBytes + (kps == 2 ? a_step : boxes * kPgABytes));
-        const int w_row = t.block * p.w_rows_per_block + (t.col_tile * (SWIGLU ? 2 : 2 * s.nb) + rank * (SWIGLU ? 1 : s.nb)) * 128;
+        const int w_row = t.block * p.w_rows_per_block +
+                          (s.narrow ? (t.col_tile * 2 + rank) * 64
+                                    : (t.col_tile * (SWIGLU ? 2 : 2 * s.nb) + rank * (SWIGLU ? 1 : s.nb)) * 128);
         const int w_step = SWIGLU ? p.up_row_offset : 128;
         const int a_row = t.row0 + rank * half;
         for (int k = g.k0; k < g.k1; k += kps) {
@@ -333,7 +340,12 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           const uint32_t bar = pair_first_cta_addr(smem_u32(&full_bar[st]));
           const uint32_t w_dst = smem_u32(smem + st * stage_bytes);
           const uint32_t a_dst = w_dst + kps * s.nb * kPgWBytes;
-          if (warp == 0) {
+          if (warp == 0 && SWIGLU && s.narrow) {
+            for (int h = 0; h < kps; ++h) {   // gate rows in the upper half of a k step's block, up rows in the lower one
+              tma_load_2d_pair(w_dst + h * kPgWBytes, &tmap_w64, bar, (k + h) * 64, w_row);
+              tma_load_2d_pair(w_dst + h * kPgWBytes + kPgWBytes / 2, &tmap_w64, bar, (k + h) * 64, w_row + w_step);
+            }
+          } else if (warp == 0) {
             for (int j = 0; j < s.nb; ++j)
               if (kps == 2)
                 tma_load_3d_pair(w_dst + j * 2 * kPgWBytes, &tmap_w2, bar, 0, w_row + j * w_step, k);
@@ -405,7 +417,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       mbar_wait(&acc_full[acc], use & 1, &abort_flag, p.status_word, 504);
       tc_fence_after_sync();
       const uint32_t d0 = tmem_base + acc * s.nb * s.tile_n + t_lane;
-      const int col_cta = (t.col_tile * (SWIGLU ? 2 : 2 * s.nb) + rank * (SWIGLU ? 1 : s.nb)) * 128;
+      const int col_cta = s.narrow ? (t.col_tile * 2 + rank) * 64
+                                   : (t.col_tile * (SWIGLU ? 2 : 2 * s.nb) + rank * (SWIGLU ? 1 : s.nb)) * 128;
       const int chunks = (t.rows + 31) >> 5;
 
       // 32 rows of one block, already final except for bias and scale: bf16 pairs to their rows
@@ -456,6 +469,35 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           if (r < live)
             __stcg(dst + static_cast<int64_t>(r) * p.n, some ? __uint_as_float(r32[r]) : 0.f);
       };
+      if (SWIGLU && s.narrow) {
+        // lane quarters 0, 1 hold gate columns, 2, 3 the up values of the same columns: these cross through shared memory
+        float* swap = reinterpret_cast<float*>(smem + kPgRing - kPgSwapBytes) + part * (32 * 64) + (q & 1) * 32 + lane;
+        for (int c = part; c < chunks; c += 2) {
+          uint32_t ra[32];
+          tmem_ld_32x32(d0 + c * 32, ra);
+          tmem_ld_wait();
+          if (q >= 2) {
+#pragma unroll
+            for (int r = 0; r < 32; ++r)
+              swap[r * 64] = __uint_as_float(ra[r]);
+          }
+          if (part == 0)
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+          else
+            asm volatile("bar.sync 3, 128;" ::: "memory");
+          if (q < 2) {
+            float a[32];
+#pragma unroll
+            for (int r = 0; r < 32; ++r)
+              a[r] = silu_f(__uint_as_float(ra[r])) * swap[r * 64];
+            store_chunk(c, col_cta, a);
+          }
+          if (part == 0)   // read before the next chunk's values overwrite them
+            asm volatile("bar.sync 2, 128;" ::: "memory");
+          else
+            asm volatile("bar.sync 3, 128;" ::: "memory");
+        }
+      } else
       for (int c = part; c < chunks; c += 2) {
         if (SWIGLU) {
           uint32_t ra[32], rb[32];
