@@ -84,11 +84,11 @@ class LLaDAAttention(nn.Module):
         if self.q_norm is not None:
             q = self.q_norm.forward_heads_(q)
         if ctx.is_full:
-            kv = self.kv_proj(hidden_states)
-            k, v = kv.split([self.kv_size, self.kv_size], dim=-1)
-            k, v = k.reshape(-1, Hkv, D), v.reshape(-1, Hkv, D)
+            # K and V come out as two tensors; the library product of both halves needed a copy of each
+            k, v = self.kv_proj.forward_gathered(hidden_states, None, hidden_states.size(0), split_col=self.kv_size)
+            k, v = k.view(-1, Hkv, D), v.view(-1, Hkv, D)
             if self.k_norm is not None:
-                k = self.k_norm.forward_heads_(k.contiguous())
+                k = self.k_norm.forward_heads_(k)
             q, k = self.rotary_emb(positions, q, k)
             self.k_cache.reset_full(k.flatten(-2, -1), md.running_seqs_tensor, seq_ids_list=md.running_seqs)
             o = self.attn(q, k, v)
