@@ -374,9 +374,13 @@ class RotaryEmbedding(nn.Module):
     def cos_sin_cache(self) -> torch.Tensor:
         return self._cos_sin_cache
 
-    def rotate(self, positions: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
+    def rotate(self, positions: torch.Tensor, x: torch.Tensor, norm: RMSNorm | None = None) -> torch.Tensor:
+        """``norm``: the per-head norm that comes before the rotation, in the same pass."""
         if self._cos_sin_cache.device != x.device:
             self._cos_sin_cache = self._cos_sin_cache.to(x.device)
+        if norm is not None:
+            return ops.head_rms_norm_rope_(x.contiguous(), norm.weight, norm.eps, positions,
+                                           self._cos_sin_cache.view(-1, x.size(-1)))
         # in place on the freshly projected [rows, heads, 128] bf16 tensor (the kernel wrapper raises otherwise)
         return ops.rope_neox_(x.contiguous(), positions, self._cos_sin_cache.view(-1, x.size(-1)))
 

@@ -81,21 +81,18 @@ class LLaDAAttention(nn.Module):
         if not ctx.is_full and salient_rows is not None and _kv_overlap() and ctx.idx_salient_row.numel():
             return self._forward_sparse_overlapped(positions, hidden_states, salient_rows)
         q = self.q_proj(hidden_states).view(-1, H, D)
-        if self.q_norm is not None:
-            q = self.q_norm.forward_heads_(q)
         if ctx.is_full:
             # K and V come out as two tensors; the library product of both halves needed a copy of each
             k, v = self.kv_proj.forward_gathered(hidden_states, None, hidden_states.size(0), split_col=self.kv_size)
             k, v = k.view(-1, Hkv, D), v.view(-1, Hkv, D)
-            if self.k_norm is not None:
-                k = self.k_norm.forward_heads_(k)
-            q, k = self.rotary_emb(positions, q, k)
+            q = self.rotary_emb.rotate(positions, q, self.q_norm)
+            k = self.rotary_emb.rotate(positions, k, self.k_norm)
             self.k_cache.reset_full(k.flatten(-2, -1), md.running_seqs_tensor, seq_ids_list=md.running_seqs)
             o = self.attn(q, k, v)
         else:
             cap = ctx.idx_salient_row.numel()   # capacity; the live count may sit on the device
             n_dev, hint = ctx.num_salient_dev, ctx.salient_hint
-            q = self.rotary_emb.rotate(positions, q)
+            q = self.rotary_emb.rotate(positions, q, self.q_norm)
             dv = None
             if cap:
                 if salient_rows is not None:
@@ -166,9 +163,7 @@ def _forward_sparse_overlapped(self, positions, hidden_states, salient_rows):
                             self.rotary_emb.cos_sin_cache.view(-1, D), ctx.cu_seqlens_k, self.k_cache.seq_start_gpu,
                             self.attn.v_cache.seq_start_gpu, md.running_seqs_tensor, self.k_cache.cache,
                             self.attn.v_cache.cache, n_dev, dv=dv)
-    if self.q_norm is not None:
-        q = self.q_norm.forward_heads_(q)
-    q = self.rotary_emb.rotate(positions, q)
+    q = self.rotary_emb.rotate(positions, q, self.q_norm)
     main.wait_stream(side)
     k_full = self.k_cache.get_seqs(md.running_seqs_tensor, allow_view=True, seq_ids_list=md.running_seqs)
     o = self.attn(q, k_full.view(-1, Hkv, D), v_new.view(cap, Hkv, D), dv=dv)

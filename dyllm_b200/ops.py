@@ -314,6 +314,23 @@ def head_rms_norm_(x: torch.Tensor, weight: torch.Tensor, eps: float, num_rows_d
     return x
 
 
+def head_rms_norm_rope_(x: torch.Tensor, weight: torch.Tensor, eps: float, positions: torch.Tensor,
+                        cos_sin: torch.Tensor) -> torch.Tensor:
+    """:func:`head_rms_norm_` followed by :func:`rope_neox_`, in one pass over ``x [rows, heads, 128]``.
+
+    ref: dyllm/model_executor/models/lladamoe.py:195-207.
+    """
+    require_cuda(x, "x", torch.bfloat16, 3)
+    require_cuda(weight, "weight", torch.bfloat16, 1)
+    require_cuda(positions, "positions", torch.int64, 1)
+    require_cuda(cos_sin, "cos_sin", torch.float32)
+    if positions.numel() < x.size(0):
+        raise RuntimeError("positions must have an entry per row")
+    call("dyllm_head_rms_norm_rope", ptr(x), ptr(weight), float(eps), ptr(positions), ptr(cos_sin), x.size(0), x.size(1),
+         x.size(2), cos_sin.size(0), stream_ptr(x.device))
+    return x
+
+
 def rope_neox_(x: torch.Tensor, positions: torch.Tensor, cos_sin: torch.Tensor, pos_idx: torch.Tensor | None = None,
                num_rows_dev: torch.Tensor | None = None) -> torch.Tensor:
     """In-place NeoX rotary embedding of ``x [rows, heads, 128]``.

@@ -386,6 +386,11 @@ int dyllm_confidence_unmask(const float* conf, const int64_t* best_token, int64_
                             int prompt_len, int block_len, int num_transfer, int64_t mask_id, int64_t* picked_pos,
                             int32_t* picked_count, void* stream);
 
+/* dyllm_head_rms_norm followed by dyllm_rope_neox (without pos_idx) in one pass, with the same roundings.  x and weight
+ * 8-byte, cos_sin 16-byte aligned.  ref: dyllm/model_executor/models/lladamoe.py:195-207. */
+int dyllm_head_rms_norm_rope(void* x, const void* weight, float eps, const int64_t* positions, const float* cos_sin,
+                             int rows, int heads, int head_dim, int max_pos, void* stream);
+
 /* NeoX-style rotary embedding applied in place to x [rows, heads, 128] (bf16): row r uses the angle
  * table row of positions[pos_idx ? pos_idx[r] : r], clamped to [0, max_pos); cos_sin is fp32
  * [max_pos, 128] = cos(64) | sin(64).  num_rows_dev (nullable) bounds the rows on the device.
