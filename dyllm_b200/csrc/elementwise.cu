@@ -97,6 +97,16 @@ add_rms_norm_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res_i
                     res_out ? res_out + row * vecs : nullptr, vecs, inv_width, eps);
 }
 
+// Cache row of every listed row (what dyllm_cache_dest_rows writes), found on the side by the blocks that walk the list.
+struct DestRows {
+  const int64_t* row_idx;      // packed row of list entry m; null = not wanted
+  const int32_t* cu;           // [batch + 1]
+  const int64_t* seq_starts;
+  const int64_t* seq_ids;
+  int batch;
+  int32_t* dest;
+};
+
 // The same arithmetic with the listed rows' normalised values also (or only) written packed in list order:
 // blocks [0, rows) handle their row (residual sum; normalised row when y_all is given), the remaining blocks
 // walk the list and write the normalised row sel_idx[m] to y_sel[m], ready to be the packed input of a
@@ -107,7 +117,7 @@ add_rms_norm_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ 
                          uint4* __restrict__ y_all, uint4* __restrict__ y_sel, uint4* __restrict__ res_out, int rows,
                          int vecs, float inv_width,
                          float eps, int x_seg_rows, int64_t x_seg_pitch_rows, const int32_t* __restrict__ sel_idx,
-                         int sel_max, const int32_t* __restrict__ sel_count_dev) {
+                         int sel_max, const int32_t* __restrict__ sel_count_dev, const DestRows d) {
   pdl_wait();      // programmatic dependent launch: nothing before this reads an earlier kernel's data
   pdl_trigger();
   if (static_cast<int>(blockIdx.x) < rows) {
@@ -119,6 +129,19 @@ add_rms_norm_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ 
   }
   const int count = sel_count_dev ? min(sel_max, *sel_count_dev) : sel_max;
   for (int m = static_cast<int>(blockIdx.x) - rows; m < count; m += static_cast<int>(gridDim.x) - rows) {
+    if (d.row_idx && threadIdx.x == 32) {
+      const int64_t r = d.row_idx[m];
+      int lo = 0, hi = d.batch;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (d.cu[mid + 1] <= r)
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      const int b = lo < d.batch ? lo : d.batch - 1;
+      d.dest[m] = static_cast<int32_t>(d.seq_starts[d.seq_ids[b]] + (r - d.cu[b]));
+    }
     int64_t row = sel_idx[m];
     row = row < 0 ? 0 : (row >= rows ? rows - 1 : row);
     const int64_t x_row = (row / x_seg_rows) * x_seg_pitch_rows + row % x_seg_rows;
@@ -471,6 +494,19 @@ int dyllm_add_rms_norm_rows(const void* x, int x_seg_rows, int64_t x_seg_pitch_r
                             const void* weight, float eps, void* y_all, void* residual_out, int rows, int width,
                             const int32_t* sel_idx, int sel_max, const int32_t* sel_count_dev, void* y_sel,
                             void* stream) {
+  return dyllm_add_rms_norm_rows_dest(x, x_seg_rows, x_seg_pitch_rows, residual_in, weight, eps, y_all, residual_out, rows,
+                                      width, sel_idx, sel_max, sel_count_dev, y_sel, nullptr, nullptr, nullptr, nullptr, 0,
+                                      nullptr, stream);
+}
+
+int dyllm_add_rms_norm_rows_dest(const void* x, int x_seg_rows, int64_t x_seg_pitch_rows, const void* residual_in,
+                                 const void* weight, float eps, void* y_all, void* residual_out, int rows, int width,
+                                 const int32_t* sel_idx, int sel_max, const int32_t* sel_count_dev, void* y_sel,
+                                 const int64_t* row_idx, const int32_t* cu_seqlens, const int64_t* seq_starts,
+                                 const int64_t* seq_ids, int batch, int32_t* dest_rows, void* stream) {
+  DYLLM_REQUIRE(!row_idx || (cu_seqlens && seq_starts && seq_ids && dest_rows && batch > 0), DYLLM_ERR_INVALID_ARGUMENT,
+                "add_rms_norm_rows: destination rows need cu_seqlens, seq_starts, seq_ids, dest_rows and a batch");
+  const DestRows d = {row_idx, cu_seqlens, seq_starts, seq_ids, batch, dest_rows};
   DYLLM_REQUIRE(rows >= 0 && width > 0 && sel_max >= 0, DYLLM_ERR_INVALID_ARGUMENT, "add_rms_norm_rows: rows %d width %d",
                 rows, width);
   DYLLM_REQUIRE(x_seg_rows > 0 && x_seg_pitch_rows >= x_seg_rows, DYLLM_ERR_INVALID_ARGUMENT,
@@ -502,7 +538,7 @@ int dyllm_add_rms_norm_rows(const void* x, int x_seg_rows, int64_t x_seg_pitch_r
 #define DYLLM_NORM_ROWS(V)                                                                                         \
   DYLLM_LAUNCH(add_rms_norm_rows_kernel<V>, grid, kNormThreads, 0, s, xp, rp, wp, yap, yp, rop, rows, vecs, inv, eps,       \
                                                             x_seg_rows, x_seg_pitch_rows, sel_idx, sel_max,       \
-                                                            sel_count_dev)
+                                                            sel_count_dev, d)
   switch (vpt) {
     case 1: DYLLM_NORM_ROWS(1); break;
     case 2: DYLLM_NORM_ROWS(2); break;

@@ -340,13 +340,13 @@ class RMSNorm(nn.Module):
         the per-head q / k norm (ref: dyllm/model_executor/models/lladamoe.py:195-207)."""
         return ops.head_rms_norm_(x, self.weight, self.eps, num_rows_dev)
 
-    def forward_rows(self, x: torch.Tensor, residual: torch.Tensor, sel_idx32: torch.Tensor, sel_count_dev=None):
+    def forward_rows(self, x: torch.Tensor, residual: torch.Tensor, sel_idx32: torch.Tensor, sel_count_dev=None, dest=None):
         """Residual add of every row, normalised values of the listed rows only, packed in list order:
         ``(y_sel, new_residual)``.  What a sparse step needs of the post-attention norm: its output feeds the
         FFN of the salient rows and nothing else (ref: dyllm/model_executor/models/llada.py:183-185)."""
         if x.dim() == 2:
             x = x.contiguous()
-        y_sel, res_out, _ = ops.add_rms_norm_rows(x, self.weight, self.eps, residual, sel_idx32, sel_count_dev)
+        y_sel, res_out, _ = ops.add_rms_norm_rows(x, self.weight, self.eps, residual, sel_idx32, sel_count_dev, dest=dest)
         return y_sel, res_out
 
     def forward_with_rows(self, x: torch.Tensor, residual: torch.Tensor | None, sel_idx32: torch.Tensor, sel_count_dev=None):
@@ -425,6 +425,17 @@ class MLPcache(nn.Module):
         return self.result()
 
 
+def salient_dest(cache_update: MLPcache):
+    """What ``RMSNorm.forward_rows`` needs to find the FFN-output cache rows of the step's salient rows on the side (None
+    with several ranks, whose exchanges place the rows themselves)."""
+    if _world_size() > 1 or sequence_sharded():
+        return None
+    ctx, md, cm = get_context(), get_metadata(), cache_update.cache_manager
+    rows_k = ctx.idx_salient_row_k if ctx.idx_salient_row_k is not None else ctx.idx_salient_row
+    out = torch.empty((ctx.idx_salient_row32.numel(),), dtype=torch.int32, device=rows_k.device)
+    return rows_k, ctx.cu_seqlens_k, cm.seq_start_gpu, md.running_seqs_tensor, out
+
+
 class LLaDAMLP(nn.Module):
     """ref: dyllm/model_executor/models/llada.py:26-43."""
 
@@ -449,12 +460,13 @@ class LLaDAMLP(nn.Module):
         return ops.swiglu_ffn(mat, self.gate_up_proj.weight, self.down_proj.weight, idx_all, num_rows=cap_total,
                               num_rows_dev=total_dev, rows_hint=hint)
 
-    def forward_salient(self, hidden: torch.Tensor, staged: bool = False) -> torch.Tensor:
+    def forward_salient(self, hidden: torch.Tensor, staged: bool = False, dest: torch.Tensor | None = None) -> torch.Tensor:
         """Sparse step on the full ``[T_q, hidden]`` activation: the salient rows are read through the step's
         index list (live count on the device) and the down projection scatters straight into the
         FFN-output cache (replaces gather_rows_2D + MLP + scatter_update,
         dyllm/model_executor/models/llada.py:184-186).  With ``staged`` the input already holds the salient
-        rows alone, packed in list order (``RMSNorm.forward_rows``)."""
+        rows alone, packed in list order (``RMSNorm.forward_rows``); ``dest``: their cache rows, when the norm has
+        found them already (``salient_dest``)."""
         ctx, md = get_context(), get_metadata()
         cap = ctx.idx_salient_row.numel()
         n_dev, hint = ctx.num_salient_dev, ctx.salient_hint
@@ -478,7 +490,8 @@ class LLaDAMLP(nn.Module):
                 with profiling.region("ffn_all_reduce", 0.0, 2.0 * rows * width * 2):
                     all_reduce_salient_rows(y, n_dev, cm, md.running_seqs_tensor, rows_k)
             else:
-                dest = ops.cache_dest_rows(rows_k, ctx.cu_seqlens_k, cm.seq_start_gpu, md.running_seqs_tensor, n_dev)
+                if dest is None:
+                    dest = ops.cache_dest_rows(rows_k, ctx.cu_seqlens_k, cm.seq_start_gpu, md.running_seqs_tensor, n_dev)
                 with profiling.region("swiglu_ffn", 6.0 * rows * width * inter, nbytes):
                     ops.swiglu_ffn(hidden, self.gate_up_proj.weight, self.down_proj.weight, idx32,
                                    num_rows=cap, num_rows_dev=n_dev, rows_hint=hint, out=cm.cache, out_row_map=dest)
@@ -560,7 +573,7 @@ class LLaDAMoESparseBlock(nn.Module):
             all_reduce_sum(y)
         return self.cache_update(y)
 
-    def forward_salient(self, hidden: torch.Tensor, staged: bool = False) -> torch.Tensor:
+    def forward_salient(self, hidden: torch.Tensor, staged: bool = False, dest: torch.Tensor | None = None) -> torch.Tensor:
         """Sparse step on the full activation: rows through the salient list, results scattered into the
         FFN-output cache (at TP/EP > 1 after the all-reduce).  With ``staged`` the input already holds the
         salient rows alone, packed in list order."""
@@ -578,7 +591,8 @@ class LLaDAMoESparseBlock(nn.Module):
                 y = self._experts(hidden, idx32, cap, n_dev, hint)
                 all_reduce_salient_rows(y, n_dev, cm, md.running_seqs_tensor, rows_k)
             else:
-                dest = ops.cache_dest_rows(rows_k, ctx.cu_seqlens_k, cm.seq_start_gpu, md.running_seqs_tensor, n_dev)
+                if dest is None:
+                    dest = ops.cache_dest_rows(rows_k, ctx.cu_seqlens_k, cm.seq_start_gpu, md.running_seqs_tensor, n_dev)
                 self._experts(hidden, idx32, cap, n_dev, hint, out=cm.cache, out_row_map=dest)
         cm.finish(md.finished_seqs)
         return self.cache_update.result()

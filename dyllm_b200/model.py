@@ -20,7 +20,7 @@ from torch import nn
 from . import ops
 from .cache_manager import CacheManager
 from .context import get_context, get_metadata
-from .layers import (Attention, ColumnParallelLinear, KVParallelLinear, LLaDAMLP, LLaDAMoESparseBlock, RMSNorm,
+from .layers import (Attention, ColumnParallelLinear, KVParallelLinear, LLaDAMLP, LLaDAMoESparseBlock, RMSNorm, salient_dest,
                      RotaryEmbedding, RowParallelLinear, _world_size, attention_scope)
 
 
@@ -201,9 +201,10 @@ def _post_attention(layer, hidden_states, residual):
         hidden_states, residual = layer.post_attention_layernorm(hidden_states, residual)
         return layer.mlp(hidden_states), residual
     if ctx.idx_salient_row32 is not None and ctx.idx_salient_row32.numel():
+        dest = salient_dest(layer.mlp.cache_update)
         staged, residual = layer.post_attention_layernorm.forward_rows(hidden_states, residual, ctx.idx_salient_row32,
-                                                                       ctx.num_salient_dev)
-        return layer.mlp.forward_salient(staged, staged=True), residual
+                                                                       ctx.num_salient_dev, dest)
+        return layer.mlp.forward_salient(staged, staged=True, dest=dest[-1] if dest else None), residual
     hidden_states, residual = layer.post_attention_layernorm(hidden_states, residual)
     return layer.mlp.forward_salient(hidden_states), residual
 

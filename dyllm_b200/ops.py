@@ -266,11 +266,14 @@ def add_rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, residual: to
 
 
 def add_rms_norm_rows(x: torch.Tensor, weight: torch.Tensor, eps: float, residual: torch.Tensor | None,
-                      sel_idx: torch.Tensor, sel_count_dev: torch.Tensor | None = None, all_rows: bool = False):
+                      sel_idx: torch.Tensor, sel_count_dev: torch.Tensor | None = None, all_rows: bool = False,
+                      dest=None):
     """RMSNorm (with the residual add) whose listed rows also come out packed in list order.  Returns
     ``(y_sel [len(sel_idx), width], new_residual [rows, width] or None, y_all [rows, width] or None)``: ``y_sel[m]`` is
     the normalised row ``sel_idx[m]`` (the packed input of a gathered GEMM), ``new_residual`` exists when a residual
-    came in, ``y_all`` only with ``all_rows``.  ``x`` as for :func:`add_rms_norm`.
+    came in, ``y_all`` only with ``all_rows``.  ``x`` as for :func:`add_rms_norm`.  ``dest``: ``(row_idx int64, cu_seqlens,
+    seq_starts, seq_ids, out int32)``; ``out[m]`` receives the cache row of ``row_idx[m]`` for the live ``m``, as
+    :func:`cache_dest_rows` gives it.
 
     ref: dyllm/model_executor/models/llada.py:176-185.
     """
@@ -297,8 +300,17 @@ def add_rms_norm_rows(x: torch.Tensor, weight: torch.Tensor, eps: float, residua
         raise RuntimeError("without a residual the normalised rows are the only output: pass all_rows=True")
     y_all = torch.empty((rows, width), dtype=x.dtype, device=x.device) if all_rows else None
     y_sel = torch.empty((sel_idx.numel(), width), dtype=x.dtype, device=x.device)
-    call("dyllm_add_rms_norm_rows", ptr(x), seg_rows, seg_pitch, ptr(residual), ptr(weight), float(eps), ptr(y_all),
-         ptr(res_out), rows, width, ptr(sel_idx), sel_idx.numel(), ptr(sel_count_dev), ptr(y_sel), stream_ptr(x.device))
+    row_idx = cu = starts = ids = dest_out = None
+    if dest is not None:
+        row_idx, cu, starts, ids, dest_out = dest
+        require_cuda(row_idx, "row_idx", torch.int64, 1)
+        require_cuda(cu, "cu_seqlens", torch.int32, 1)
+        require_cuda(dest_out, "dest", torch.int32, 1)
+        if row_idx.numel() < sel_idx.numel() or dest_out.numel() < sel_idx.numel():
+            raise RuntimeError("row_idx and dest must have an entry per listed row")
+    call("dyllm_add_rms_norm_rows_dest", ptr(x), seg_rows, seg_pitch, ptr(residual), ptr(weight), float(eps), ptr(y_all),
+         ptr(res_out), rows, width, ptr(sel_idx), sel_idx.numel(), ptr(sel_count_dev), ptr(y_sel), ptr(row_idx), ptr(cu),
+         ptr(starts), ptr(ids), ids.numel() if ids is not None else 0, ptr(dest_out), stream_ptr(x.device))
     return y_sel, res_out, y_all
 
 

@@ -354,6 +354,15 @@ int dyllm_add_rms_norm_rows(const void* x, int x_seg_rows, int64_t x_seg_pitch_r
                             const int32_t* sel_idx, int sel_max, const int32_t* sel_count_dev, void* y_sel,
                             void* stream);
 
+/* The same call that also writes dest_rows[m], m < min(sel_max, *sel_count_dev): the cache row of packed row row_idx[m], as
+ * dyllm_cache_dest_rows does (which fills the rest with -1; here it stays as it is).  row_idx null = not wanted.
+ * ref: dyllm/csrc/cache/cache_kernels.cu:398-421. */
+int dyllm_add_rms_norm_rows_dest(const void* x, int x_seg_rows, int64_t x_seg_pitch_rows, const void* residual_in,
+                                 const void* weight, float eps, void* y_all, void* residual_out, int rows, int width,
+                                 const int32_t* sel_idx, int sel_max, const int32_t* sel_count_dev, void* y_sel,
+                                 const int64_t* row_idx, const int32_t* cu_seqlens, const int64_t* seq_starts,
+                                 const int64_t* seq_ids, int batch, int32_t* dest_rows, void* stream);
+
 /* RMSNorm over the head_dim values of every (row, head) of x [rows, heads, 128] (bf16), in place:
  * x = bf16( bf16(x * rsqrt(mean(x^2) + eps)) * weight ), weight bf16 [128].  num_rows_dev (nullable) bounds the
  * rows on the device.  The per-head q / k normalisation of LLaDA-MoE.
