@@ -122,7 +122,9 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def stream_ptr(device: torch.device | None = None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    # the raw handle: building a torch.cuda.Stream object on every call is a tenth of a host-driven step
+    index = device.index if device is not None else None
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def call(name: str, *args) -> None:

@@ -672,6 +672,8 @@ class Attention(nn.Module):
         estimate is that constant and no host state is touched (steps captured into a CUDA graph)."""
         if fixed:
             return min(fixed, capacity)
+        if not profiling.enabled():
+            return capacity      # no launch is shaped by the estimate any more: read back for the region timings only
         if self._hint_host is None:
             self._hint_host = torch.zeros(1, dtype=torch.int32).pin_memory()
             self._hint_event = torch.cuda.Event()
