@@ -36,7 +36,7 @@ SIGNATURES: dict[str, tuple] = {
     "dyllm_cache_scatter_update": (I, [P, P, P, P, I, P, P, I, I, P, I, I, P]),
     "dyllm_gathered_linear_workspace_bytes": (Z, [I, I, I]),
     "dyllm_gathered_linear": (I, [P, I, I, c_int64, P, I, P, I, P, I, P, c_int64, P, c_int64, I, P, P, P, Z, I, I, P]),
-    "dyllm_gathered_linear_bias": (I, [P, I, I, c_int64, P, I, P, I, P, I, P, c_int64, P, c_int64, I, P, P, P, Z, I, I, P, I, P]),
+    "dyllm_gathered_linear_bias": (I, [P, I, I, c_int64, P, I, P, I, P, I, P, c_int64, P, c_int64, I, P, P, P, Z, I, I, P, I, I, P]),
     "dyllm_swiglu_ffn_workspace_bytes": (Z, [I, I, I]),
     "dyllm_swiglu_ffn": (I, [P, I, I, c_int64, P, I, P, I, P, P, I, P, c_int64, P, P, Z, I, I, P]),
     "dyllm_cache_dest_rows": (I, [P, P, P, P, I, I, P, P, P]),

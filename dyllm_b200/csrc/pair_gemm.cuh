@@ -63,7 +63,8 @@ struct PairGemmParams {
   int split_col;                // multiple of 128
   const int32_t* out_row_map;   // destination row per row (negative = drop); null = identity
   const float* row_scale;       // multiplier per row; null = 1
-  const __nv_bfloat16* bias;    // [n] added to the rounded result (bf16 + bf16); null = none
+  const __nv_bfloat16* bias;    // [n]; null = none
+  int bias_fp32;                // 1: added to the fp32 sum, one rounding; 0: to the rounded result (bf16 + bf16)
   float* partial;               // partial sums [parts][kSplitRows][n] of a cut k range; null = never cut
   int* tickets;                 // arrival counters, zero between launches
   int split_slots;              // CTAs that gemm.cuh would have resident: the number of parts follows from it
@@ -434,14 +435,21 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         const int col = col_block + q * 32 + lane;
         const int col2 = col & ~1;
         __nv_bfloat162 bias = __floats2bfloat162_rn(0.f, 0.f);
-        if (p.bias && col2 < p.n)
+        float own_bias = 0.f;
+        if (p.bias && col2 < p.n) {
           bias = *reinterpret_cast<const __nv_bfloat162*>(p.bias + col2);
+          own_bias = odd ? __bfloat162float(bias.y) : __bfloat162float(bias.x);
+        }
         const bool second = p.out2 && col_block >= p.split_col;
         __nv_bfloat16* base = second ? p.out2 + (col2 - p.split_col) : p.out + col2;
         const int64_t ld = second ? p.ldc2 : p.ldc;
 #pragma unroll
         for (int r = 0; r < 32; r += 2) {
           float v0 = v[r], v1 = v[r + 1];
+          if (p.bias && p.bias_fp32) {
+            v0 += own_bias;
+            v1 += own_bias;
+          }
           if (p.row_scale) {
             v0 *= __shfl_sync(0xffffffffu, scale, r);
             v1 *= __shfl_sync(0xffffffffu, scale, r + 1);
@@ -449,7 +457,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
           const int row = __shfl_sync(0xffffffffu, dest, r + (odd ? 1 : 0));
           __nv_bfloat162 h = __floats2bfloat162_rn(odd ? got : v0, odd ? v1 : got);
-          if (p.bias)
+          if (p.bias && !p.bias_fp32)
             h = __hadd2(h, bias);
           if (row >= 0 && col2 < p.n)
             *reinterpret_cast<__nv_bfloat162*>(base + row * ld) = h;
@@ -584,10 +592,15 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                   a[2] += v[z][x].z;
                   a[3] += v[z][x].w;
                 }
+                if (p.bias && p.bias_fp32) {
+#pragma unroll
+                  for (int z = 0; z < 4; ++z)
+                    a[z] += __bfloat162float(p.bias[col + z]);
+                }
                 __nv_bfloat162 h[2];
                 h[0] = __floats2bfloat162_rn(a[0] * scale, a[1] * scale);
                 h[1] = __floats2bfloat162_rn(a[2] * scale, a[3] * scale);
-                if (p.bias) {
+                if (p.bias && !p.bias_fp32) {
 #pragma unroll
                   for (int z = 0; z < 2; ++z)
                     h[z] = __hadd2(h[z], *reinterpret_cast<const __nv_bfloat162*>(p.bias + col + 2 * z));

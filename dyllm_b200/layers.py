@@ -247,7 +247,7 @@ class ColumnParallelLinear(LinearBase):
         return _project(x, self.weight, self.bias)
 
     def forward_gathered(self, x: torch.Tensor, idx32: torch.Tensor | None, num_rows: int, num_rows_dev=None,
-                         rows_hint: int = 0, split_col: int = 0, out=None, few_rows_ctas: int = 0):
+                         rows_hint: int = 0, split_col: int = 0, out=None, few_rows_ctas: int = 0, bias_fp32: bool = False):
         """``self(x[idx])`` on the tcgen05 GEMM; ``num_rows`` may be a capacity with the live count on the
         device.  ``idx32`` None: ``x`` already holds the rows packed in list order.  With ``split_col`` the
         output columns are returned as two tensors (K and V halves); ``out`` may bring them (a pair)."""
@@ -260,7 +260,8 @@ class ColumnParallelLinear(LinearBase):
         else:
             out, out2 = torch.empty((num_rows, n_out), dtype=x.dtype, device=x.device), None
         ops.gathered_linear(x, self.weight, idx32, num_rows=num_rows, num_rows_dev=num_rows_dev, rows_hint=rows_hint,
-                            out=out, out2=out2, split_col=split_col, few_rows_ctas=few_rows_ctas, bias=self.bias)
+                            out=out, out2=out2, split_col=split_col, few_rows_ctas=few_rows_ctas, bias=self.bias,
+                            bias_fp32=bias_fp32)
         return (out, out2) if split_col else out
 
 

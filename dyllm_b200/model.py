@@ -82,8 +82,10 @@ class LLaDAAttention(nn.Module):
             return self._forward_sparse_overlapped(positions, hidden_states, salient_rows)
         q = self.q_proj(hidden_states).view(-1, H, D)
         if ctx.is_full:
-            # K and V come out as two tensors; the library product of both halves needed a copy of each
-            k, v = self.kv_proj.forward_gathered(hidden_states, None, hidden_states.size(0), split_col=self.kv_size)
+            # K and V come out as two tensors (the library product of both halves needed a copy of each); a bias joins the
+            # fp32 sum, as in the library product
+            k, v = self.kv_proj.forward_gathered(hidden_states, None, hidden_states.size(0), split_col=self.kv_size,
+                                                 bias_fp32=True)
             k, v = k.view(-1, Hkv, D), v.view(-1, Hkv, D)
             q = self.rotary_emb.rotate(positions, q, self.q_norm)
             k = self.rotary_emb.rotate(positions, k, self.k_norm)

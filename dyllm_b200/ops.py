@@ -126,9 +126,11 @@ def gathered_linear(x: torch.Tensor, weight: torch.Tensor, idx: torch.Tensor | N
                     num_rows: int | None = None, num_rows_dev: torch.Tensor | None = None, rows_hint: int = 0,
                     out: torch.Tensor | None = None, out2: torch.Tensor | None = None, split_col: int = 0,
                     out_row_map: torch.Tensor | None = None, row_scale: torch.Tensor | None = None, a_mode: int = -1,
-                    tile_n: int = 0, few_rows_ctas: int = 0, bias: torch.Tensor | None = None) -> torch.Tensor:
+                    tile_n: int = 0, few_rows_ctas: int = 0, bias: torch.Tensor | None = None,
+                    bias_fp32: bool = False) -> torch.Tensor:
     """``out[map[m]] = scale[m] * (x[idx[m]] @ weight.T) + bias`` on the tcgen05 tensor cores.  ``few_rows_ctas``: SMs to keep
-    to while the live rows fit one row tile (a call that runs beside another stream's kernel); 0 = all.
+    to while the live rows fit one row tile (a call that runs beside another stream's kernel); 0 = all.  ``bias_fp32``:
+    the bias joins the fp32 sum (one rounding) instead of the bf16 result.
 
     ref: dyllm/model_executor/models/llada.py:108 (``kv_proj(hidden_states[idx_salient_row])``).
     """
@@ -151,7 +153,7 @@ def gathered_linear(x: torch.Tensor, weight: torch.Tensor, idx: torch.Tensor | N
     ws = _gemm_workspace(need, x.device)
     call("dyllm_gathered_linear_bias", ptr(x), x.size(0), x.size(1), x.stride(0), ptr(idx), num_rows, ptr(num_rows_dev),
          int(rows_hint), ptr(weight), n_out, ptr(out), out.stride(0), ptr(out2), out2.stride(0) if out2 is not None else 0,
-         int(split_col), ptr(out_row_map), ptr(row_scale), ptr(ws), ws.numel(), a_mode, tile_n, ptr(bias), int(few_rows_ctas), stream_ptr(x.device))
+         int(split_col), ptr(out_row_map), ptr(row_scale), ptr(ws), ws.numel(), a_mode, tile_n, ptr(bias), int(bias_fp32), int(few_rows_ctas), stream_ptr(x.device))
     return out
 
 

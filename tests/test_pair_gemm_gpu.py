@@ -117,6 +117,10 @@ def test_bias_equals_a_separate_addition(cuda_device, rows):
     _status_ok()
     assert torch.equal(k, plain[:, :384] + bias[:384])
     assert torch.equal(v, plain[:, 384:] + bias[384:])
+    once = ops.gathered_linear(x, w, bias=bias, bias_fp32=True)
+    want = x.double() @ w.double().t() + bias.double()
+    # one rounding of an fp32 sum of 512 products: half an ulp and what the sum is off by
+    assert bool(((once.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all())
 
 
 @pytest.mark.parametrize("rows", [1, 100, 128, 129, 200, 256, 300, 512, 513])
