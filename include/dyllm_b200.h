@@ -295,7 +295,7 @@ size_t dyllm_moe_ffn_workspace_bytes(int max_rows, int top_k, int num_local_expe
  * (0 <= e < num_local_experts) of  topk_weights[m, j] * down_e( silu(x Wg_e^T) * (x Wu_e^T) ),
  * x = x[idx[m]].  w1: bf16 [num_local_experts, 2 * inter, hidden] (gate rows first), w2: bf16
  * [num_local_experts, hidden, inter].  Rows without a local expert get zeros.  The (row, slot) pairs are
- * grouped by expert on the device, each group padded to 128-row tiles; the routing weight is applied
+ * grouped by expert on the device (row tiles of at most 256 rows per expert); the routing weight is applied
  * in the down projection's epilogue and the slot sum runs in fp32 in slot order.  With
  * expert_start = 0 and all experts local this is the reference's fused_experts; a contiguous expert
  * range gives one rank's share under expert parallelism (the caller all-reduces the outputs).
