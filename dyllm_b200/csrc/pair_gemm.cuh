@@ -131,11 +131,12 @@ __device__ __forceinline__ bool pg_schedule(const PairGemmParams& p, bool swiglu
       s.row_tiles = (s.m + s.tile_n - 1) / s.tile_n;
     }
   // One or two weight blocks per CTA: two need fewer operand bytes per flop, one gives twice the tiles to fill the waves
-  // with.  A wave of one-block tiles takes ~0.6 of the time of a wave of two-block tiles at 256 rows (62 B/clk of operands
-  // against 47), and half at few rows.
+  // with.  A wave of one-block tiles takes ~2/3 of the time of a wave of two-block tiles at 256 rows (62 B/clk of operands
+  // against 47), and half at few rows.  (K = 12288, 4096 columns: 5000 rows 600 us in five waves of one block, 450 us in
+  // three of two; 3277 rows three against two waves, which is even.)
   const int t1 = s.row_tiles * ((p.n + 255) >> 8), t2 = s.row_tiles * ((p.n + 511) >> 9);
   const int w1 = (t1 * s.parts + s.pairs - 1) / s.pairs, w2 = (t2 * s.parts + s.pairs - 1) / s.pairs;
-  s.nb = swiglu ? (s.narrow ? 1 : 2) : (p.row_tiles ? (s.tile_n > 128 ? 2 : 1) : (w1 * 3 <= w2 * 5 ? 1 : 2));
+  s.nb = swiglu ? (s.narrow ? 1 : 2) : (p.row_tiles ? (s.tile_n > 128 ? 2 : 1) : (w1 * 2 <= w2 * 3 ? 1 : 2));
   const int cols = swiglu ? pair_cols : s.nb * 256;
   s.col_tiles = (p.n + cols - 1) / cols;
   s.units = s.row_tiles * s.col_tiles * s.parts;
