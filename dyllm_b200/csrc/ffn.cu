@@ -116,6 +116,15 @@ Plan make_plan(bool swiglu, int M, int hint, int n, int K, int tile_n, bool can_
   return plan;
 }
 
+// Into how many parts the pair kernel cuts the k range of a plain product: the parts that gathered_gemm_kernel would cut it
+// into at this launch's row estimate, so that both add up the same sums whatever the count on the device turns out to be.
+void set_cut(PairGemmParams& q, int rows_hint) {
+  const Plan plan = make_plan(false, q.M, rows_hint, q.n, q.K, 0, q.partial != nullptr, true);
+  q.max_parts = plan.splits;
+  q.cut_col_tiles = q.n / plan.tile_n;
+  q.cut_slots = plan.slots;
+}
+
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Which of the two kernels runs a call that names neither a tile width nor a_mode 1 (both give the same bits).  The pair
@@ -366,6 +375,7 @@ int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64
     q.bias = static_cast<const __nv_bfloat16*>(bias);
     q.bias_fp32 = bias_fp32;
     q.partial = partial;
+    set_cut(q, rows_hint);
     q.one_tile_pairs = few_rows_ctas > 0 ? (few_rows_ctas + 1) / 2 : 0;
     return launch_pair_gemm(false, q, g.a, g.a_rows, lda, weight, out_features, s);
   }
@@ -448,6 +458,7 @@ int dyllm_swiglu_ffn(const void* x, int x_rows, int hidden, int64_t ldx, const i
     q.out = static_cast<__nv_bfloat16*>(out);
     q.ldc = ldo;
     q.out_row_map = out_row_map;
+    set_cut(q, rows_hint);
     return launch_pair_gemm(false, q, inter_buf, static_cast<int>(padded), inter, w_down, hidden, s);
   }
   GemmParams g2 = {};

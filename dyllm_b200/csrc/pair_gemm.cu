@@ -71,7 +71,6 @@ int launch_pair_gemm(bool swiglu, const PairGemmParams& p_in, const void* a, int
   pairs = pairs < 1 ? 1 : (pairs > kPgMaxPairs ? kPgMaxPairs : pairs);
   p.status_word = device_status_word();
   p.tickets = p.partial ? pair_tickets(p.partial) : nullptr;
-  p.split_slots = 2 * sm_count();
   if (!p.tickets)
     p.partial = nullptr;
   // boxes of one k step (64 columns) and, as 3-D boxes [k step][row][column], of two

@@ -15,7 +15,8 @@
 // Work split: tiles are dealt to the pairs in turn (groups of eight row tiles, so that the tiles in flight share weights
 // and activations in L2).  Few rows of a plain product cut the k range into up to four parts: fp32 partial sums go to the
 // workspace and the CTA that finishes a tile last adds them in k order (the same sum whoever is last).  The number of
-// parts is effective_splits() of gemm.cuh whatever the tile shape here, so both kernels give the same bits.  (Equal shares
+// parts is that of gemm.cuh for the launch's row estimate (set_cut() in ffn.cu) and the live count, whatever the tile shape
+// here, so both kernels give the same bits.  (Equal shares
 // per pair over all sizes, so that the last wave is always full, were measured too: 280 us against 289 us for a 3277 x
 // 4096 x 12288 product, nothing at few rows, and other sums.)
 //
@@ -68,7 +69,9 @@ struct PairGemmParams {
   int bias_fp32;                // 1: added to the fp32 sum, one rounding; 0: to the rounded result (bf16 + bf16)
   float* partial;               // partial sums [parts][kSplitRows][n] of a cut k range; null = never cut
   int* tickets;                 // arrival counters, zero between launches
-  int split_slots;              // CTAs that gemm.cuh would have resident: the number of parts follows from it
+  int max_parts;                // parts of a cut k range: effective_splits() of these three and the live count
+  int cut_col_tiles;
+  int cut_slots;
   int one_tile_pairs;           // pairs that work when all rows fit one row tile (0 = all)
   int* status_word;
 };
@@ -120,8 +123,8 @@ __device__ __forceinline__ bool pg_schedule(const PairGemmParams& p, bool swiglu
   s.narrow = swiglu && 2 * s.row_tiles * ((p.n + 255) >> 8) <= s.pairs;
   const int pair_cols = s.narrow ? 128 : 256;
   s.parts = 1;
-  if (!swiglu && !p.row_tiles && p.partial && s.m <= kSplitRows)
-    s.parts = effective_splits((s.m + 127) >> 7, p.n >> 6, p.split_slots, kMaxSplits, s.kt);
+  if (!swiglu && !p.row_tiles && p.partial && p.max_parts > 1 && s.m <= kSplitRows)
+    s.parts = effective_splits((s.m + kGemmBM - 1) / kGemmBM, p.cut_col_tiles, p.cut_slots, p.max_parts, s.kt);
   s.part_kt = (s.kt + s.parts - 1) / s.parts;
   // More and lower row tiles (the weights come from L2 the second time) give more pairs work, too.
   if (!p.row_tiles)

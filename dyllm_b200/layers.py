@@ -669,12 +669,11 @@ class Attention(nn.Module):
     def _next_hint(self, count_dev: torch.Tensor, capacity: int, fixed: int = 0) -> int:
         """Estimate of the salient count this layer has just produced: its value from the previous step
         (read back asynchronously, never waited for), or the capacity when none has arrived yet.  The
-        estimate only shapes launches; kernels take the true count from the device.  With ``fixed`` the
+        estimate shapes launches (kernel, grid, into how many parts k is cut: with them the order of the fp32 sums);
+        kernels take the true count from the device.  With ``fixed`` the
         estimate is that constant and no host state is touched (steps captured into a CUDA graph)."""
         if fixed:
             return min(fixed, capacity)
-        if not profiling.enabled():
-            return capacity      # no launch is shaped by the estimate any more: read back for the region timings only
         if self._hint_host is None:
             self._hint_host = torch.zeros(1, dtype=torch.int32).pin_memory()
             self._hint_event = torch.cuda.Event()
