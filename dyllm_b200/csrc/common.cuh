@@ -34,9 +34,12 @@ int sm_count();
 // on a wait stores a non-zero code here; the host entry point that launched it reports
 // DYLLM_ERR_DEVICE_TIMEOUT on its next status query.
 int* device_status_word();            // device pointer (per device), zero-initialised
-// Per-device arrival counters for split-K output tiles (kSplitTicketCount ints, zero between launches).
-constexpr int kSplitTicketCount = 4096;
-int* split_tickets();
+// Arrival counters of the output tiles of a product that is cut along k: kTicketCount words in the call's own workspace,
+// right before the partial sums, so calls with different workspaces never meet.  A workspace comes as it is, so a counter
+// cannot be expected to be zero: a word counts only if it carries the number of this launch (see open_counter).
+constexpr int kTicketCount = 1024;
+constexpr size_t kTicketBytes = kTicketCount * sizeof(unsigned long long);
+unsigned long long next_launch_id();   // another one for every call in this process; the three lowest bits are zero
 int read_and_clear_device_status();   // synchronises the given stream's device; used by tests
 
 // Programmatic dependent launch (off with DYLLM_PDL=0 in the environment).

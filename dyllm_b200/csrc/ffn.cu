@@ -177,7 +177,8 @@ __global__ void cache_dest_rows_kernel(const int64_t* __restrict__ row_idx, cons
 
 // a_mode: 0 = A rows m0..m0+127 by one TMA box (A dense or already staged), 1 = TMA gather4 through
 // p.a_idx.  n is the number of output columns per weight block (the intermediate size for SWIGLU).
-// tile_n: 64, 128 or (many rows, no SwiGLU) 256 (0 = choose).  `partial` enables split-K for the non-SwiGLU GEMM.
+// tile_n: 64, 128 or (many rows, no SwiGLU) 256 (0 = choose).  `partial` enables split-K for the non-SwiGLU GEMM; the
+// arrival counters (kTicketBytes) lie right before it.
 int launch_gathered_gemm(bool swiglu, int a_mode, int tile_n, const GemmParams& p_in, int64_t lda, const void* b,
                          int64_t b_total_rows, int n, int rows_hint, float* partial, cudaStream_t stream) {
   GemmParams p = p_in;
@@ -203,9 +204,13 @@ int launch_gathered_gemm(bool swiglu, int a_mode, int tile_n, const GemmParams& 
   p.status_word = device_status_word();
   p.n_total = n;
   p.partial = plan.splits > 1 ? partial : nullptr;
-  p.split_tickets = split_tickets();
-  if (!p.split_tickets || static_cast<int64_t>(plan.grid.x) * (kSplitRows / kGemmBM) > kSplitTicketCount)
+  // tiles are cut only while they fill less than half of the CTA slots, so there are at most sms of them
+  if (static_cast<int64_t>(plan.grid.x) * (kSplitRows / kGemmBM) > kTicketCount)
     p.partial = nullptr;   // no counters for this many tiles: every CTA runs its whole k range
+  if (p.partial) {
+    p.split_tickets = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(p.partial) - kTicketBytes);
+    p.launch_id = next_launch_id();
+  }
   p.split_rows = kSplitRows;
   p.split_slots = plan.slots;
 
@@ -265,7 +270,7 @@ extern "C" {
 size_t dyllm_gathered_linear_workspace_bytes(int max_rows, int in_features, int out_features) {
   if (max_rows <= 0 || in_features <= 0 || out_features <= 0)
     return 0;
-  return align_up(padded_rows(max_rows) * static_cast<size_t>(in_features) * 2, 1024) +
+  return align_up(padded_rows(max_rows) * static_cast<size_t>(in_features) * 2, 1024) + kTicketBytes +
          static_cast<size_t>(kMaxSplits) * kSplitRows * out_features * sizeof(float);
 }
 
@@ -274,7 +279,7 @@ size_t dyllm_swiglu_ffn_workspace_bytes(int max_rows, int hidden, int inter) {
     return 0;
   const size_t padded = padded_rows(max_rows);
   return align_up(padded * static_cast<size_t>(hidden) * 2, 1024) +
-         align_up(padded * static_cast<size_t>(inter) * 2, 1024) +
+         align_up(padded * static_cast<size_t>(inter) * 2, 1024) + kTicketBytes +
          static_cast<size_t>(kMaxSplits) * kSplitRows * hidden * sizeof(float);
 }
 
@@ -358,7 +363,7 @@ int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64
   g.split_col = out2 ? split_col : 0;
   g.out_row_map = out_row_map;
   g.row_scale = row_scale;
-  float* partial = have_ws ? reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + stage_bytes) : nullptr;
+  float* partial = have_ws ? reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + stage_bytes + kTicketBytes) : nullptr;
   if (bias || (mode == 0 && tile_n == 0 && !few_tiles(false, out_features, in_features, num_rows, num_rows_dev, rows_hint))) {
     PairGemmParams q = {};
     q.m_count_dev = num_rows_dev;
@@ -406,7 +411,7 @@ int dyllm_swiglu_ffn(const void* x, int x_rows, int hidden, int64_t ldx, const i
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   void* staged = ws;
   uint8_t* inter_buf = ws + align_up(padded * static_cast<size_t>(hidden) * 2, 1024);
-  float* partial = reinterpret_cast<float*>(inter_buf + align_up(padded * static_cast<size_t>(inter) * 2, 1024));
+  float* partial = reinterpret_cast<float*>(inter_buf + align_up(padded * static_cast<size_t>(inter) * 2, 1024) + kTicketBytes);
 
   GemmParams g1 = {};
   g1.a = static_cast<const __nv_bfloat16*>(x);

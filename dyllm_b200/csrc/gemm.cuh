@@ -40,7 +40,8 @@ struct GemmParams {
   int64_t ldc2;
   int split_col;
   float* partial;              // split-K: fp32 [gridDim.y][split_rows][n_total]; null = no split-K
-  int* split_tickets;          // split-K: arrival counter per (row tile, column tile), zero between launches
+  unsigned long long* split_tickets;   // split-K: arrival counter per (row tile, column tile)
+  unsigned long long launch_id;        // tells this launch's counter words from whatever the workspace held
   int split_rows;              // split-K is used only while the live row count is <= split_rows
   int split_slots;             // CTAs the device runs at once; the live split count is derived from it
   int n_total;                 // output columns (row pitch of `partial`)
@@ -79,6 +80,27 @@ __host__ __device__ __forceinline__ int effective_splits(int live_tiles, int n_t
   s = s > max_splits ? max_splits : s;
   s = s > num_kt ? num_kt : s;
   return s < 1 ? 1 : s;
+}
+
+// Counter of a tile that is cut into 2 .. 4 parts, in a workspace that nobody has cleared.  Every part makes the word this
+// launch's first (open_counter: its upper 61 bits become the launch's number; an uninitialised word carries it already with
+// a probability of 2^-61), which one thread does while the tile's products run; arriving is then a single addition (a
+// compare-and-swap at that point, with the other parts arriving at the same time, cost 2 us per product).
+__device__ __forceinline__ void open_counter(unsigned long long* word, unsigned long long launch_id) {
+  unsigned long long seen = *reinterpret_cast<volatile unsigned long long*>(word);
+  while (((seen ^ launch_id) >> 3) != 0) {
+    const unsigned long long was = atomicCAS(word, seen, launch_id);
+    if (was == seen)
+      return;
+    seen = was;      // another part has opened it in between
+  }
+}
+// True for the part that arrives last, which leaves a zero: a launch that a graph replays finds the word as if new.
+__device__ __forceinline__ bool last_to_arrive(unsigned long long* word, int parts) {
+  if ((atomicAdd(word, 1ull) & 7) != static_cast<unsigned long long>(parts - 1))
+    return false;
+  *reinterpret_cast<volatile unsigned long long*>(word) = 0;
+  return true;
 }
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
@@ -241,6 +263,8 @@ gathered_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     for (int mt = blockIdx.z; mt * BM < m_count; mt += gridDim.z, ++ti) {
       const int acc = MT == 1 ? (ti & 1) : 0;
       const uint32_t use = MT == 1 ? (ti >> 1) : ti;
+      if (!SWIGLU && MT == 1 && write_partial && threadIdx.x == 64)
+        open_counter(p.split_tickets + mt * gridDim.x + n_tile, p.launch_id);
       mbar_wait(&tmem_full_bar[acc], use & 1, &abort_flag, p.status_word, 204);
       tc_fence_after_sync();
 #pragma unroll 1
@@ -318,11 +342,7 @@ gathered_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         __threadfence();
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (threadIdx.x == 64) {
-          int* ticket = p.split_tickets + mt * gridDim.x + n_tile;
-          const int t = atomicAdd(ticket, 1);
-          last_split = (t == splits - 1) ? 1 : 0;
-          if (t == splits - 1)
-            *ticket = 0;   // every split has arrived: ready for the next launch
+          last_split = last_to_arrive(p.split_tickets + mt * gridDim.x + n_tile, splits) ? 1 : 0;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (last_split) {

@@ -7,30 +7,6 @@ namespace dyllm {
 
 namespace {
 
-// Arrival counters of the tiles that are cut along k: zero between launches (the last arrival resets its counter).  Calls
-// that may run at the same time have different workspaces, so the workspace picks the set of counters; two workspaces
-// share a set with a probability of 1 / 256.
-constexpr int kPgTicketSets = 256;
-constexpr int kPgTickets = 384;                  // two per cut tile, of which there are at most an eighth of the CTA slots
-__device__ int g_pair_tickets[kPgTicketSets * kPgTickets] = {0};
-std::atomic<int*> g_pair_tickets_ptr[64];
-
-int* pair_tickets(const void* workspace) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
-    return nullptr;
-  int* base = g_pair_tickets_ptr[dev].load(std::memory_order_acquire);
-  if (!base) {
-    void* sym = nullptr;
-    if (cudaGetSymbolAddress(&sym, g_pair_tickets) != cudaSuccess)
-      return nullptr;
-    base = static_cast<int*>(sym);
-    g_pair_tickets_ptr[dev].store(base, std::memory_order_release);   // every thread finds the same address
-  }
-  const uint64_t h = (reinterpret_cast<uintptr_t>(workspace) >> 8) * 0x9E3779B97F4A7C15ull;
-  return base + (h >> 56) * kPgTickets;
-}
-
 template <bool SWIGLU>
 int launch(const CUtensorMap (&t)[6], const PairGemmParams& p, int pairs, cudaStream_t stream) {
   auto kernel = pair_gemm_kernel<SWIGLU>;
@@ -52,7 +28,7 @@ int launch(const CUtensorMap (&t)[6], const PairGemmParams& p, int pairs, cudaSt
 }  // namespace
 
 // `a` holds a_rows rows of pitch lda (p.M dense rows, or the rows that p.row_tiles list); `w` holds w_total_rows rows
-// of p.K.  p.status_word and p.tickets are filled in here.
+// of p.K.  p.status_word, p.tickets and p.launch_id are filled in here.
 int launch_pair_gemm(bool swiglu, const PairGemmParams& p_in, const void* a, int a_rows, int64_t lda, const void* w,
                      int64_t w_total_rows, cudaStream_t stream) {
   PairGemmParams p = p_in;
@@ -70,9 +46,13 @@ int launch_pair_gemm(bool swiglu, const PairGemmParams& p_in, const void* a, int
   int pairs = sm_count() / 2;
   pairs = pairs < 1 ? 1 : (pairs > kPgMaxPairs ? kPgMaxPairs : pairs);
   p.status_word = device_status_word();
-  p.tickets = p.partial ? pair_tickets(p.partial) : nullptr;
-  if (!p.tickets)
-    p.partial = nullptr;
+  // a cut launch has at most 2 * pairs tiles (each part of a tile is a piece of work, and tiles are only made smaller while
+  // the pieces do not fill the pairs): two words for each fit
+  static_assert(4 * kPgMaxPairs <= kTicketCount, "arrival counters of the cut tiles");
+  if (p.partial) {
+    p.tickets = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(p.partial) - kTicketBytes);
+    p.launch_id = next_launch_id();
+  }
   // boxes of one k step (64 columns) and, as 3-D boxes [k step][row][column], of two
   CUtensorMap t[6];
   int rc = encode_tmap_2d_bf16(&t[0], w, w_total_rows, p.K, p.K, 128, 64, true);

@@ -41,7 +41,7 @@
 
 #include <cooperative_groups.h>
 
-#include "gemm.cuh"   // effective_splits()
+#include "gemm.cuh"   // effective_splits(), open_counter(), last_to_arrive()
 
 namespace dyllm {
 
@@ -68,7 +68,8 @@ struct PairGemmParams {
   const __nv_bfloat16* bias;    // [n]; null = none
   int bias_fp32;                // 1: added to the fp32 sum, one rounding; 0: to the rounded result (bf16 + bf16)
   float* partial;               // partial sums [parts][kSplitRows][n] of a cut k range; null = never cut
-  int* tickets;                 // arrival counters, zero between launches
+  unsigned long long* tickets;  // arrival counters of cut tiles, two per tile (one per CTA of a pair)
+  unsigned long long launch_id;
   int max_parts;                // parts of a cut k range: effective_splits() of these three and the live count
   int cut_col_tiles;
   int cut_slots;
@@ -420,6 +421,9 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const PgTile t = pg_tile(p, s, g.tile);
       const int acc = accs == 2 ? (seg & 1) : 0;
       const uint32_t use = accs == 2 ? (seg >> 1) : seg;
+      const bool cut = !SWIGLU && s.parts > 1;
+      if (cut && threadIdx.x == 128)
+        open_counter(p.tickets + g.tile * 2 + rank, p.launch_id);
       mbar_wait(&acc_full[acc], use & 1, &abort_flag, p.status_word, 504);
       tc_fence_after_sync();
       const uint32_t d0 = tmem_base + acc * s.nb * s.tile_n + t_lane;
@@ -468,7 +472,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             *reinterpret_cast<__nv_bfloat162*>(base + row * ld) = h;
         }
       };
-      const bool cut = !SWIGLU && s.parts > 1;
       const int64_t part_floats = static_cast<int64_t>(kSplitRows) * p.n;
       auto keep_chunk = [&](int c, int col_block, const uint32_t (&r32)[32]) {   // partial sums of one block
         const int col = col_block + q * 32 + lane;
@@ -549,13 +552,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       if (cut) {
         __threadfence();
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (threadIdx.x == 128) {
-          int* ticket = p.tickets + g.tile * 2 + rank;
-          const int n = atomicAdd(ticket, 1);
-          last_part = n == s.parts - 1 ? 1 : 0;
-          if (n == s.parts - 1)
-            *ticket = 0;   // every part has arrived: ready for the next launch
-        }
+        if (threadIdx.x == 128)
+          last_part = last_to_arrive(p.tickets + g.tile * 2 + rank, s.parts) ? 1 : 0;
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (last_part) {
           __threadfence();

@@ -11,6 +11,13 @@ from . import _lib as _lib_mod
 from ._lib import call, load, ptr, require_cuda, stream_ptr
 
 
+def _scratch(nbytes: int, device) -> torch.Tensor:
+    """Workspace of one call.  It comes from, and goes back to, the caching allocator in the order of the current stream (or
+    of the graph that is being captured), so calls on different streams, from different threads and in graphs that outlive
+    the call never find another one's row staging, partial sums or arrival counters in it."""
+    return torch.empty(max(nbytes, 16), dtype=torch.uint8, device=device)
+
+
 def context_stats(c_old: torch.Tensor, c_new: torch.Tensor, out: torch.Tensor | None = None,
                   accumulate: bool = False) -> torch.Tensor:
     """[dot(new, old), |new|^2, |old|^2] per row in fp32.
@@ -54,18 +61,6 @@ class SalientSelection:
         self.cu_salientlens, self.count, self.mask = cu_salientlens, count, mask
 
 
-_workspaces: dict = {}
-
-
-def _select_workspace(rows: int, device: torch.device) -> torch.Tensor:
-    need = load().dyllm_salient_select_workspace_bytes(rows)
-    ws = _workspaces.get(device)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(max(need, 4096), dtype=torch.uint8, device=device)
-        _workspaces[device] = ws
-    return ws
-
-
 def salient_select(stats: torch.Tensor, threshold: float, cu_seqlens_q: torch.Tensor,
                    cu_promptlens: torch.Tensor | None = None, want_mask: bool = False,
                    want_idx32: bool = True) -> SalientSelection:
@@ -88,7 +83,7 @@ def salient_select(stats: torch.Tensor, threshold: float, cu_seqlens_q: torch.Te
     cu_sal = torch.empty((batch + 1,), dtype=torch.int32, device=dev)
     count = torch.empty((1,), dtype=torch.int32, device=dev)
     mask = torch.empty((rows,), dtype=torch.bool, device=dev) if want_mask else None
-    ws = _select_workspace(rows, dev)
+    ws = _scratch(load().dyllm_salient_select_workspace_bytes(rows), dev)
     call("dyllm_salient_select", ptr(stats), rows, float(threshold), ptr(cu_seqlens_q), batch, ptr(cu_promptlens),
          ptr(idx), ptr(idx32), ptr(idx_k), ptr(cu_sal), ptr(count), ptr(mask), ptr(ws), ws.numel(), stream_ptr(dev))
     return SalientSelection(idx, idx32, idx_k, cu_sal, count, mask)
@@ -107,19 +102,6 @@ def cache_dest_rows(row_idx: torch.Tensor, cu_seqlens: torch.Tensor, seq_starts:
     call("dyllm_cache_dest_rows", ptr(row_idx), ptr(cu_seqlens), ptr(seq_starts), ptr(seq_ids), seq_ids.numel(), n,
          ptr(num_rows_dev), ptr(dest), stream_ptr(row_idx.device))
     return dest
-
-
-_gemm_workspaces: dict = {}
-
-
-def _gemm_workspace(nbytes: int, device) -> torch.Tensor:
-    """One shared scratch tensor per device for the row staging, the FFN intermediate and split-K sums
-    (kernels on one stream use it one after the other)."""
-    ws = _gemm_workspaces.get(device)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _gemm_workspaces[device] = ws
-    return ws
 
 
 def gathered_linear(x: torch.Tensor, weight: torch.Tensor, idx: torch.Tensor | None = None,
@@ -150,7 +132,7 @@ def gathered_linear(x: torch.Tensor, weight: torch.Tensor, idx: torch.Tensor | N
     if num_rows == 0:
         return out
     need = load().dyllm_gathered_linear_workspace_bytes(num_rows, x.size(1), n_out)
-    ws = _gemm_workspace(need, x.device)
+    ws = _scratch(need, x.device)
     call("dyllm_gathered_linear_bias", ptr(x), x.size(0), x.size(1), x.stride(0), ptr(idx), num_rows, ptr(num_rows_dev),
          int(rows_hint), ptr(weight), n_out, ptr(out), out.stride(0), ptr(out2), out2.stride(0) if out2 is not None else 0,
          int(split_col), ptr(out_row_map), ptr(row_scale), ptr(ws), ws.numel(), a_mode, tile_n, ptr(bias), int(bias_fp32), int(few_rows_ctas), stream_ptr(x.device))
@@ -179,7 +161,7 @@ def swiglu_ffn(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, i
         out = torch.empty((num_rows, hidden), dtype=torch.bfloat16, device=x.device)
     if num_rows == 0:
         return out
-    ws = _gemm_workspace(load().dyllm_swiglu_ffn_workspace_bytes(num_rows, hidden, inter), x.device)
+    ws = _scratch(load().dyllm_swiglu_ffn_workspace_bytes(num_rows, hidden, inter), x.device)
     call("dyllm_swiglu_ffn", ptr(x), x.size(0), hidden, x.stride(0), ptr(idx), num_rows, ptr(num_rows_dev),
          int(rows_hint), ptr(w_gate_up), ptr(w_down), inter, ptr(out), out.stride(0), ptr(out_row_map), ptr(ws),
          ws.numel(), a_mode, tile_n, stream_ptr(x.device))
@@ -438,7 +420,7 @@ def moe_ffn(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, topk_weights: t
         out = torch.empty((num_rows, hidden), dtype=torch.bfloat16, device=x.device)
     if num_rows == 0:
         return out
-    ws = _gemm_workspace(load().dyllm_moe_ffn_workspace_bytes(num_rows, top_k, e_local, hidden, inter), x.device)
+    ws = _scratch(load().dyllm_moe_ffn_workspace_bytes(num_rows, top_k, e_local, hidden, inter), x.device)
     call("dyllm_moe_ffn", ptr(x), x.size(0), hidden, x.stride(0), ptr(idx), num_rows, ptr(num_rows_dev), int(rows_hint),
          ptr(topk_weights), ptr(topk_ids), top_k, ptr(w1), ptr(w2), e_local, int(expert_start), inter, ptr(out),
          out.stride(0), ptr(out_row_map), ptr(ws), ws.numel(), stream_ptr(x.device))

@@ -151,8 +151,8 @@ int dyllm_cache_scatter_update(void* cache, const void* new_rows, const int64_t*
  * x.  tile_n = 64, 128, 256 (plain product with many rows only) or 0 (choose).
  * ---------------------------------------------------------------------------------------------- */
 
-/* Bytes of workspace dyllm_gathered_linear needs for up to max_rows rows (row staging + split-K
- * partial sums).  Without a workspace the call still works with a_mode 1 or idx == null. */
+/* Bytes of workspace dyllm_gathered_linear needs for up to max_rows rows (row staging, split-K
+ * arrival counters and partial sums).  Without a workspace the call still works with a_mode 1 or idx == null. */
 size_t dyllm_gathered_linear_workspace_bytes(int max_rows, int in_features, int out_features);
 
 /* out[map[m]] = scale[m] * (x[idx[m]] W^T), m < min(num_rows, *num_rows_dev).  idx null = identity,
@@ -160,9 +160,9 @@ size_t dyllm_gathered_linear_workspace_bytes(int max_rows, int in_features, int 
  * output columns >= split_col (a multiple of 128) go to out2[.., column - split_col] instead (used to
  * write K and V of the fused K/V projection into two tensors).  in_features % 64 == 0,
  * out_features % 64 == 0.  Tiles that would leave many SMs idle are cut along k (deterministic: fp32 partial sums go to
- * the workspace, and the CTA that finishes an output tile last adds them in k order inside the same launch).  Arrival
- * counters live in a small array inside the library, chosen by the workspace: calls that share a workspace must not
- * overlap on the GPU (issue them on one stream), nor calls that name a tile width or a_mode 1.
+ * the workspace, and the CTA that finishes an output tile last adds them in k order inside the same launch).  The arrival
+ * counters lie in the workspace too (which need not be cleared): calls that share a workspace must not overlap on the GPU
+ * (issue them on one stream); calls with different workspaces may.
  * ref: dyllm/model_executor/models/llada.py:108 (kv_proj(hidden_states[idx_salient_row])),
  *      dyllm/model_executor/layers/linear.py:50-51. */
 int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ldx, const int32_t* idx,
