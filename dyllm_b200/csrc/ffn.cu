@@ -340,6 +340,8 @@ int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64
   int mode = a_mode;
   DYLLM_REQUIRE(!bias || (mode == 0 && tile_n == 0), DYLLM_ERR_UNSUPPORTED,
                 "gathered_linear: a bias needs a_mode 0 and no tile width");
+  DYLLM_REQUIRE((reinterpret_cast<uintptr_t>(bias) & 1) == 0, DYLLM_ERR_INVALID_ARGUMENT,
+                "gathered_linear: a bias must be 2-byte aligned");
   DYLLM_REQUIRE(few_rows_ctas >= 0, DYLLM_ERR_INVALID_ARGUMENT, "gathered_linear: few_rows_ctas %d", few_rows_ctas);
   if (idx && a_mode == 0) {
     int rc = stage_rows(x, ldx, idx, x_rows, workspace, in_features, num_rows, num_rows_dev, rows_hint, s);

@@ -65,7 +65,7 @@ struct PairGemmParams {
   int split_col;                // multiple of 128
   const int32_t* out_row_map;   // destination row per row (negative = drop); null = identity
   const float* row_scale;       // multiplier per row; null = 1
-  const __nv_bfloat16* bias;    // [n]; null = none
+  const __nv_bfloat16* bias;    // [n], at any element; null = none
   int bias_fp32;                // 1: added to the fp32 sum, one rounding; 0: to the rounded result (bf16 + bf16)
   float* partial;               // partial sums [parts][kSplitRows][n] of a cut k range; null = never cut
   unsigned long long* tickets;  // arrival counters of cut tiles, two per tile (one per CTA of a pair)
@@ -446,7 +446,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         __nv_bfloat162 bias = __floats2bfloat162_rn(0.f, 0.f);
         float own_bias = 0.f;
         if (p.bias && col2 < p.n) {
-          bias = *reinterpret_cast<const __nv_bfloat162*>(p.bias + col2);
+          bias = __halves2bfloat162(p.bias[col2], p.bias[col2 + 1]);   // a bias may start at any element
           own_bias = odd ? __bfloat162float(bias.y) : __bfloat162float(bias.x);
         }
         const bool second = p.out2 && col_block >= p.split_col;
@@ -606,7 +606,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 if (p.bias && !p.bias_fp32) {
 #pragma unroll
                   for (int z = 0; z < 2; ++z)
-                    h[z] = __hadd2(h[z], *reinterpret_cast<const __nv_bfloat162*>(p.bias + col + 2 * z));
+                    h[z] = __hadd2(h[z], __halves2bfloat162(p.bias[col + 2 * z], p.bias[col + 2 * z + 1]));
                 }
                 *reinterpret_cast<uint2*>(base + dest * ld) = *reinterpret_cast<const uint2*>(h);
               }

@@ -187,9 +187,18 @@ def set_projection_backend(name: str) -> None:
     _projection_backend = name
 
 
+def _epilogue_bias(bias: torch.Tensor | None) -> torch.Tensor | None:
+    """The bias if the GEMM's epilogue can add it; any other (another type, strided) is added to the result."""
+    return bias if bias is not None and bias.dtype == torch.bfloat16 and bias.is_contiguous() else None
+
+
 def _project(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None) -> torch.Tensor:
     if _projection_backend == "tcgen05" and x.is_cuda and x.dim() == 2 and x.size(0) > 0:
-        return ops.gathered_linear(x.contiguous(), weight, None, num_rows=x.size(0), rows_hint=x.size(0), bias=bias)
+        fused = _epilogue_bias(bias)
+        y = ops.gathered_linear(x.contiguous(), weight, None, num_rows=x.size(0), rows_hint=x.size(0), bias=fused)
+        if bias is not fused:
+            y += bias
+        return y
     return F.linear(x, weight, bias)
 
 
@@ -259,9 +268,14 @@ class ColumnParallelLinear(LinearBase):
             out2 = torch.empty((num_rows, n_out - split_col), dtype=x.dtype, device=x.device)
         else:
             out, out2 = torch.empty((num_rows, n_out), dtype=x.dtype, device=x.device), None
+        fused = _epilogue_bias(self.bias)
         ops.gathered_linear(x, self.weight, idx32, num_rows=num_rows, num_rows_dev=num_rows_dev, rows_hint=rows_hint,
-                            out=out, out2=out2, split_col=split_col, few_rows_ctas=few_rows_ctas, bias=self.bias,
+                            out=out, out2=out2, split_col=split_col, few_rows_ctas=few_rows_ctas, bias=fused,
                             bias_fp32=bias_fp32)
+        if self.bias is not fused:
+            out += self.bias[: out.size(1)]
+            if out2 is not None:
+                out2 += self.bias[out.size(1):]
         return (out, out2) if split_col else out
 
 

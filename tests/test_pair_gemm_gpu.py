@@ -136,3 +136,46 @@ def test_same_bits_as_the_kernel_with_named_tiles(cuda_device, rows, k, n):
     if rows <= 256:      # beyond, the other kernel has one CTA per SM and cuts less
         assert torch.equal(got, want)
     _close(got, x.double() @ w.double().t(), "plain")
+
+
+@pytest.mark.parametrize("offset", [0, 1, 3])
+@pytest.mark.parametrize("rows,k,n", [(40, 4096, 1024), (300, 512, 1088)])
+def test_bias_at_any_element(cuda_device, rows, k, n, offset):
+    """A bias that is a view at an odd offset, in the epilogue of whole tiles (300 rows) and of tiles cut along k (40)."""
+    from dyllm_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, w, bias = _randn(g, rows, k), _randn(g, n, k, scale=0.05), _randn(g, n + 8)[offset:offset + n]
+    plain = ops.gathered_linear(x, w, bias=torch.zeros_like(bias), bias_fp32=True)
+    got = ops.gathered_linear(x, w, bias=bias)
+    once = ops.gathered_linear(x, w, bias=bias, bias_fp32=True)
+    _status_ok()
+    assert torch.equal(got, plain + bias)
+    assert torch.equal(once, ops.gathered_linear(x, w, bias=bias.clone(), bias_fp32=True))
+
+
+@pytest.mark.parametrize("make", [lambda b: b.float(), lambda b: torch.stack([b, b], 1)[:, 0]])
+def test_layer_adds_a_bias_that_the_epilogue_cannot(cuda_device, make):
+    """fp32 or strided: added to the bf16 result, as an in-place addition does it."""
+    from dyllm_b200 import layers
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    lin = layers.ColumnParallelLinear(512, 1024, bias=True).to("cuda", torch.bfloat16)
+    lin.weight.data = _randn(g, 1024, 512, scale=0.05)
+    bias = _randn(g, 1024)
+    x = _randn(g, 70, 512)
+    with torch.inference_mode():
+        lin.bias = None
+        plain = lin.forward_gathered(x, None, 70)
+        lin.bias = torch.nn.Parameter(make(bias), requires_grad=False)
+        want = plain.clone()
+        want += lin.bias
+        assert torch.equal(lin.forward_gathered(x, None, 70), want)
+        k, v = lin.forward_gathered(x, None, 70, split_col=256)
+        assert torch.equal(torch.cat([k, v], 1), want)
+        layers.set_projection_backend("tcgen05")
+        try:
+            assert torch.equal(lin(x), want)
+        finally:
+            layers.set_projection_backend("cublas")
+    _status_ok()
