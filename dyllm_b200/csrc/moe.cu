@@ -101,7 +101,9 @@ route_rows(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __re
     const int m = m0 + warp;
     if (warp < R && m < n) {
       float* s_logits = s_all[warp];
-      // softmax over the experts, then top-k by repeated arg-max (lowest index wins ties)
+      // softmax over the experts, then top-k by repeated arg-max (lowest index wins ties).  NaN (a logit that is NaN or
+      // +inf) ranks below every number and above the experts already taken (-1), so that a pick is an expert always; the
+      // sum, hence every weight of such a row, is NaN.
       float mx = -3.0e38f;
       for (int e = lane; e < num_experts; e += 32)
         mx = fmaxf(mx, s_logits[e]);
@@ -125,7 +127,7 @@ route_rows(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __re
         float best = -1.f;
         int best_e = 0x7fffffff;
         for (int e = lane; e < num_experts; e += 32) {
-          const float v = s_logits[e];
+          const float v = isnan(s_logits[e]) ? -0.5f : s_logits[e];
           if (v > best) {
             best = v;
             best_e = e;

@@ -91,3 +91,34 @@ def test_moe_gathered_rows_device_count_and_scatter(cuda_device):
     untouched = torch.ones(300, dtype=torch.bool)
     untouched[dest[:live].long()] = False
     assert bool((out.cpu()[untouched] == 3.0).all())
+
+
+@pytest.mark.parametrize("rows", [6, 700])
+def test_router_row_without_numbers_keeps_to_its_experts(cuda_device, rows):
+    """Rows that hold NaN or whose logits overflow to infinity, next to finite ones (one and four rows per block): expert ids
+    stay in range and differ within the row, the weights are NaN and reach the output, the other rows are as without them."""
+    from dyllm_b200 import _lib, ops
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    hidden, inter, experts, top_k = 256, 64, 64, 8
+    x = torch.randn(rows, hidden, generator=g, device="cuda").bfloat16()
+    wr = (torch.randn(experts, hidden, generator=g, device="cuda") * 0.1).bfloat16()
+    w1 = (torch.randn(experts, 2 * inter, hidden, generator=g, device="cuda") * 0.05).bfloat16()
+    w2 = (torch.randn(experts, hidden, inter, generator=g, device="cuda") * 0.05).bfloat16()
+    want_w, want_ids = ops.moe_route(x, wr, top_k)
+    want = ops.moe_ffn(x, w1, w2, want_w, want_ids)
+    bad = torch.tensor([1, 4, rows - 1], device="cuda")
+    broken = x.clone()
+    broken[1, 7] = float("nan")                 # every logit NaN
+    broken[4] = float("inf")                    # inf - inf
+    broken[rows - 1, 0] = float("inf")          # logits of both infinities
+    got_w, got_ids = ops.moe_route(broken, wr, top_k)
+    got = ops.moe_ffn(broken, w1, w2, got_w, got_ids)
+    assert _lib.load().dyllm_device_status() == 0
+    assert bool(((got_ids >= 0) & (got_ids < experts)).all())
+    assert bool((got_ids.sort(dim=1).values.diff(dim=1) > 0).all())
+    assert bool(got_w[bad].isnan().all()) and bool(got[bad].isnan().all())
+    good = torch.ones(rows, dtype=torch.bool, device="cuda")
+    good[bad] = False
+    assert torch.equal(got_w[good], want_w[good]) and torch.equal(got_ids[good], want_ids[good])
+    assert torch.equal(got[good], want[good])
