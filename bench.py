@@ -561,7 +561,7 @@ def run_ours(args, cfg, tau):
                "stage_seconds_per_layer_step": stages}
     cfg_d = config_dict(cfg, tau, world, args)
     cfg_d["tp_exchange"] = exchange
-    cfg_d["all_row_projections"] = args.projection
+    cfg_d["all_row_projections"] = "cublas" if args.projection == "default" else args.projection
     cfg_d["dense_step_attention"] = args.dense_attention
     if world > 1:
         cfg_d["layout"] = layout
@@ -610,8 +610,9 @@ def main():
     ap.add_argument("--layers", type=int, default=0, help="debug only: fewer layers marks the line invalid")
     ap.add_argument("--denoise-steps", type=int, default=0, help="debug only")
     ap.add_argument("--full-steps", type=int, default=None, help="debug only: dense steps per generation")
-    ap.add_argument("--projection", default="cublas", choices=["cublas", "tcgen05"],
-                    help="GEMM of the all-row q / o projections: cuBLAS (default) or this package's tcgen05 GEMM")
+    ap.add_argument("--projection", default="default", choices=["default", "cublas", "tcgen05"],
+                    help="GEMM of the all-row q / o projections: cuBLAS (default) or this package's tcgen05 GEMM; with "
+                         "\"cublas\" the dense steps' K/V projection runs there too")
     ap.add_argument("--dense-attention", default="sdpa", choices=["tcgen05", "sdpa"],
                     help="attention of the dense steps: torch SDPA (default) or this package's exact-attention kernel")
     ap.add_argument("--no-cpu-baseline", action="store_true")

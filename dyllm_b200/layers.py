@@ -175,14 +175,15 @@ def _gathered_ffn(ffn_shard, x: torch.Tensor, idx32, cap_local: int, count_dev, 
     return out
 
 
-# Which GEMM runs the all-row projections (q_proj, o_proj, dense-step kv_proj): "cublas" (F.linear; plain library
-# GEMMs, the default) or "tcgen05" (this package's gathered GEMM on every row, 256-row tiles).
-_projection_backend = "cublas"
+# Which GEMM runs the all-row projections (q_proj, o_proj, dense-step kv_proj): "cublas" (F.linear; plain library GEMMs),
+# "tcgen05" (this package's GEMM on every row) or "default" (library GEMMs for q_proj and o_proj, this package's for the
+# dense-step kv_proj, whose two halves it writes as two tensors).
+_projection_backend = "default"
 
 
 def set_projection_backend(name: str) -> None:
     global _projection_backend
-    if name not in ("cublas", "tcgen05"):
+    if name not in ("default", "cublas", "tcgen05"):
         raise ValueError(f"unknown projection backend {name!r}")
     _projection_backend = name
 
@@ -200,6 +201,21 @@ def _project(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None) -
             y += bias
         return y
     return F.linear(x, weight, bias)
+
+
+def as_defined(module, cls, *names: str) -> bool:
+    """``module`` runs ``cls``'s own methods of these names: not overridden in a subclass, not replaced on the object.  The
+    shorter ways through a layer that pass such a method by, or call it with an argument of this package's, are taken only
+    then."""
+    return all(getattr(type(module), n, None) is getattr(cls, n) and n not in module.__dict__ for n in names)
+
+
+def unhooked(module: nn.Module) -> bool:
+    """No hook would see a call of ``module``."""
+    g = nn.modules.module
+    return not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks
+                or g._global_backward_pre_hooks)
 
 
 def divide(numerator: int, denominator: int) -> int:

@@ -330,11 +330,12 @@ def _bench_projection(args, backend):
     dev = torch.device("cuda")
     x = torch.randn(B * L, HID, device=dev).bfloat16()
     w = (torch.randn(HID, HID, device=dev) * 0.02).bfloat16()
+    before = layers._projection_backend
     layers.set_projection_backend(backend)
     try:
         ms = time_launches(lambda: layers._project(x, w, None), args.iters, args.flush)
     finally:
-        layers.set_projection_backend("cublas")
+        layers.set_projection_backend(before)
     return ms, 2.0 * B * L * HID * HID, "F"
 
 

@@ -17,11 +17,11 @@ import os
 import torch
 from torch import nn
 
-from . import ops
+from . import layers, ops
 from .cache_manager import CacheManager
 from .context import get_context, get_metadata
 from .layers import (Attention, ColumnParallelLinear, KVParallelLinear, LLaDAMLP, LLaDAMoESparseBlock, RMSNorm, salient_dest,
-                     RotaryEmbedding, RowParallelLinear, _world_size, attention_scope)
+                     RotaryEmbedding, RowParallelLinear, _world_size, as_defined, attention_scope, unhooked)
 
 
 @dataclass
@@ -39,6 +39,15 @@ class LLaDAShape:
     rope_theta: float = 500000.0
     max_sequence_length: int = 4096
     mask_token_id: int = 126336
+
+
+def _norm_and_rotate(rotary, positions: torch.Tensor, x: torch.Tensor, norm) -> torch.Tensor:
+    """Per-head norm (if there is one) and rotary embedding: one pass where both are this package's own."""
+    if norm is None:
+        return rotary.rotate(positions, x)
+    if as_defined(norm, RMSNorm, "forward_heads_") and as_defined(rotary, RotaryEmbedding, "rotate"):
+        return rotary.rotate(positions, x, norm)
+    return rotary.rotate(positions, norm.forward_heads_(x.contiguous()))
 
 
 class LLaDAAttention(nn.Module):
@@ -82,19 +91,31 @@ class LLaDAAttention(nn.Module):
             return self._forward_sparse_overlapped(positions, hidden_states, salient_rows)
         q = self.q_proj(hidden_states).view(-1, H, D)
         if ctx.is_full:
-            # K and V come out as two tensors (the library product of both halves needed a copy of each); a bias joins the
-            # fp32 sum, as in the library product
-            k, v = self.kv_proj.forward_gathered(hidden_states, None, hidden_states.size(0), split_col=self.kv_size,
-                                                 bias_fp32=True)
-            k, v = k.view(-1, Hkv, D), v.view(-1, Hkv, D)
-            q = self.rotary_emb.rotate(positions, q, self.q_norm)
-            k = self.rotary_emb.rotate(positions, k, self.k_norm)
+            kv_proj = self.kv_proj
+            if layers._projection_backend == "default" and unhooked(kv_proj) and \
+                    as_defined(kv_proj, ColumnParallelLinear, "forward", "forward_gathered"):
+                # K and V come out as two tensors (the product of both halves needs a copy of each); a bias joins the fp32
+                # sum, as in the library product
+                k, v = kv_proj.forward_gathered(hidden_states, None, hidden_states.size(0), split_col=self.kv_size,
+                                                bias_fp32=True)
+            else:
+                k, v = kv_proj(hidden_states).split([self.kv_size, self.kv_size], dim=-1)
+            k, v = k.reshape(-1, Hkv, D), v.reshape(-1, Hkv, D)
+            if unhooked(self.rotary_emb) and as_defined(self.rotary_emb, RotaryEmbedding, "forward"):
+                q = _norm_and_rotate(self.rotary_emb, positions, q, self.q_norm)
+                k = _norm_and_rotate(self.rotary_emb, positions, k, self.k_norm)
+            else:
+                if self.q_norm is not None:
+                    q = self.q_norm.forward_heads_(q)
+                if self.k_norm is not None:
+                    k = self.k_norm.forward_heads_(k.contiguous())
+                q, k = self.rotary_emb(positions, q, k)
             self.k_cache.reset_full(k.flatten(-2, -1), md.running_seqs_tensor, seq_ids_list=md.running_seqs)
             o = self.attn(q, k, v)
         else:
             cap = ctx.idx_salient_row.numel()   # capacity; the live count may sit on the device
             n_dev, hint = ctx.num_salient_dev, ctx.salient_hint
-            q = self.rotary_emb.rotate(positions, q, self.q_norm)
+            q = _norm_and_rotate(self.rotary_emb, positions, q, self.q_norm)
             dv = None
             if cap:
                 if salient_rows is not None:
@@ -127,9 +148,7 @@ def _kv_overlap() -> bool:
     """The K/V branch of a sparse step (projection of the salient rows, K/V cache update) runs on a second stream
     beside the query projection, whose cuBLAS kernel leaves SMs idle in its last wave (DYLLM_KV_OVERLAP=0: one
     stream).  Not with this package's own GEMM for the all-row projections, which leaves no SM idle."""
-    from . import layers
-
-    return os.environ.get("DYLLM_KV_OVERLAP", "1") != "0" and layers._projection_backend == "cublas"
+    return os.environ.get("DYLLM_KV_OVERLAP", "1") != "0" and layers._projection_backend != "tcgen05"
 
 
 def _forward_sparse_overlapped(self, positions, hidden_states, salient_rows):
@@ -154,10 +173,10 @@ def _forward_sparse_overlapped(self, positions, hidden_states, salient_rows):
     side.wait_event(forked)
     # Beside a query projection of many rows the few salient rows' product keeps to 40 SMs, about what the library
     # kernel's last wave leaves idle: the weights stream in under it either way.  A short one has no such tail.
-    ctas = 40 if hidden_states.size(0) >= 2048 else 0
+    ctas = 40 if hidden_states.size(0) >= 2048 and as_defined(self.kv_proj, ColumnParallelLinear, "forward_gathered") else 0
     with torch.cuda.stream(side):
         self.kv_proj.forward_gathered(salient_rows, None, cap, n_dev, hint, split_col=self.kv_size, out=(k_new, v_new),
-                                      few_rows_ctas=ctas)
+                                      **({"few_rows_ctas": ctas} if ctas else {}))
         k3 = k_new.view(cap, Hkv, D)
         if self.k_norm is not None:
             k3 = self.k_norm.forward_heads_(k3, n_dev)
@@ -165,7 +184,7 @@ def _forward_sparse_overlapped(self, positions, hidden_states, salient_rows):
                             self.rotary_emb.cos_sin_cache.view(-1, D), ctx.cu_seqlens_k, self.k_cache.seq_start_gpu,
                             self.attn.v_cache.seq_start_gpu, md.running_seqs_tensor, self.k_cache.cache,
                             self.attn.v_cache.cache, n_dev, dv=dv)
-    q = self.rotary_emb.rotate(positions, q, self.q_norm)
+    q = _norm_and_rotate(self.rotary_emb, positions, q, self.q_norm)
     main.wait_stream(side)
     k_full = self.k_cache.get_seqs(md.running_seqs_tensor, allow_view=True, seq_ids_list=md.running_seqs)
     o = self.attn(q, k_full.view(-1, Hkv, D), v_new.view(cap, Hkv, D), dv=dv)
@@ -203,10 +222,15 @@ def _post_attention(layer, hidden_states, residual):
         hidden_states, residual = layer.post_attention_layernorm(hidden_states, residual)
         return layer.mlp(hidden_states), residual
     if ctx.idx_salient_row32 is not None and ctx.idx_salient_row32.numel():
-        dest = salient_dest(layer.mlp.cache_update)
-        staged, residual = layer.post_attention_layernorm.forward_rows(hidden_states, residual, ctx.idx_salient_row32,
-                                                                       ctx.num_salient_dev, dest)
-        return layer.mlp.forward_salient(staged, staged=True, dest=dest[-1] if dest else None), residual
+        norm, mlp, dest = layer.post_attention_layernorm, layer.mlp, None
+        if as_defined(norm, RMSNorm, "forward_rows") and (as_defined(mlp, LLaDAMLP, "forward_salient")
+                                                          or as_defined(mlp, LLaDAMoESparseBlock, "forward_salient")):
+            dest = salient_dest(mlp.cache_update)
+        if dest is None:
+            staged, residual = norm.forward_rows(hidden_states, residual, ctx.idx_salient_row32, ctx.num_salient_dev)
+            return mlp.forward_salient(staged, staged=True), residual
+        staged, residual = norm.forward_rows(hidden_states, residual, ctx.idx_salient_row32, ctx.num_salient_dev, dest)
+        return mlp.forward_salient(staged, staged=True, dest=dest[-1]), residual
     hidden_states, residual = layer.post_attention_layernorm(hidden_states, residual)
     return layer.mlp.forward_salient(hidden_states), residual
 
