@@ -370,6 +370,16 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           }
         }
       }
+      // The first CTA's commits arrive at the second CTA's barriers, too: every stage is seen released before this CTA may
+      // end, so that none arrives at the shared memory of a CTA that has left.
+      if (warp == 0)
+        for (int i = 0; i < stages; ++i) {
+          mbar_wait(&empty_bar[st], ph ^ 1, &abort_flag, p.status_word, 506);
+          if (++st == stages) {
+            st = 0;
+            ph ^= 1;
+          }
+        }
     }
     __syncwarp();
   } else if (warp == 1) {
