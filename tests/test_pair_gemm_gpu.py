@@ -27,22 +27,33 @@ def _randn(g, *shape, scale=1.0):
     return (torch.randn(*shape, generator=g, device="cuda") * scale).bfloat16()
 
 
+def _pair(x, w, **kw):
+    """The product on the pair kernel, whatever its size: a bias takes a call there, and zeros added in fp32 change nothing."""
+    from dyllm_b200 import ops
+
+    return ops.gathered_linear(x, w, bias=torch.zeros(w.size(0), dtype=torch.bfloat16, device="cuda"), bias_fp32=True, **kw)
+
+
 @pytest.mark.parametrize("rows", [1, 31, 33, 96, 128, 129, 160, 256, 257, 513, 1100])
-@pytest.mark.parametrize("k,n", [(64, 64), (192, 192), (1024, 576), (12288, 512), (320, 4096)])
+@pytest.mark.parametrize("k,n", [(64, 64), (192, 192), (1024, 576), (12288, 512), (320, 4096), (4096, 4096), (2112, 2304)])
 def test_plain_product(cuda_device, rows, k, n):
+    """As the package chooses the kernel (the last two sizes are the pair kernel's at any row count), and the pair kernel by
+    force: its row tiles, parts of an odd number of k steps (2112), an empty last part (320)."""
     from dyllm_b200 import ops
 
     g = torch.Generator(device="cuda").manual_seed(rows * 7 + k + n)
     x, w = _randn(g, rows, k), _randn(g, n, k, scale=0.05)
-    got = ops.gathered_linear(x, w)
-    again = ops.gathered_linear(x, w)
-    _status_ok()
-    _close(got, x.double() @ w.double().t(), "plain")
-    assert torch.equal(got, again), "the sum of a cut tile does not depend on which CTA arrives last"
+    want = x.double() @ w.double().t()
+    for product in (ops.gathered_linear, _pair):
+        got = product(x, w)
+        again = product(x, w)
+        _status_ok()
+        _close(got, want, "plain")
+        assert torch.equal(got, again), "the sum of a cut tile does not depend on which CTA arrives last"
 
 
 @pytest.mark.parametrize("rows", [1, 40, 129, 256, 300, 700])
-@pytest.mark.parametrize("hidden,inter", [(64, 64), (256, 192), (4096, 320), (512, 1536), (2048, 4096)])
+@pytest.mark.parametrize("hidden,inter", [(64, 64), (256, 192), (4096, 320), (512, 1536), (2048, 4096), (2304, 2112)])
 def test_swiglu_ffn(cuda_device, rows, hidden, inter):
     from dyllm_b200 import ops
 
@@ -126,15 +137,17 @@ def test_bias_equals_a_separate_addition(cuda_device, rows):
 @pytest.mark.parametrize("rows", [1, 100, 128, 129, 200, 256, 300, 512, 513])
 @pytest.mark.parametrize("k,n", [(320, 256), (4096, 1024), (1088, 4096)])
 def test_same_bits_as_the_kernel_with_named_tiles(cuda_device, rows, k, n):
-    """The k range is cut into the same parts as by the 64-column tiles, summed in the same order."""
+    """The k range is cut into the same parts as by the tile width that the other kernel takes for this many rows, summed in
+    the same order."""
     from dyllm_b200 import ops
 
     g = torch.Generator(device="cuda").manual_seed(rows + k)
     x, w = _randn(g, rows, k), _randn(g, n, k, scale=0.05)
-    got, want = ops.gathered_linear(x, w), ops.gathered_linear(x, w, tile_n=64)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tile = 128 if -(-rows // 128) * (n // 128) >= sms * 3 // 4 else 64
+    got, want = _pair(x, w), ops.gathered_linear(x, w, tile_n=tile)
     _status_ok()
-    if rows <= 256:      # beyond, the other kernel has one CTA per SM and cuts less
-        assert torch.equal(got, want)
+    assert torch.equal(got, want)
     _close(got, x.double() @ w.double().t(), "plain")
 
 
