@@ -42,7 +42,7 @@ constexpr size_t kTicketBytes = kTicketCount * sizeof(unsigned long long);
 unsigned long long next_launch_id();   // another one for every call in this process; the three lowest bits are zero
 int read_and_clear_device_status();   // synchronises the given stream's device; used by tests
 
-// Programmatic dependent launch (off with DYLLM_PDL=0 in the environment).
+// Programmatic dependent launch (on with DYLLM_PDL=1 in the environment).
 bool pdl_enabled();
 
 #ifdef __CUDACC__

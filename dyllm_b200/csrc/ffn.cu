@@ -304,15 +304,15 @@ int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ld
                           const float* row_scale, void* workspace, size_t workspace_bytes, int a_mode, int tile_n,
                           void* stream) {
   return dyllm_gathered_linear_bias(x, x_rows, in_features, ldx, idx, num_rows, num_rows_dev, rows_hint, weight,
-                                      out_features, out, ldo, out2, ldo2, split_col, out_row_map, row_scale, workspace,
-                                      workspace_bytes, a_mode, tile_n, nullptr, 0, 0, stream);
+                                    out_features, out, ldo, out2, ldo2, split_col, out_row_map, row_scale, workspace,
+                                    workspace_bytes, a_mode, tile_n, nullptr, 0, 0, stream);
 }
 
 int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64_t ldx, const int32_t* idx,
-                                 int num_rows, const int32_t* num_rows_dev, int rows_hint, const void* weight,
-                                 int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
-                                 const int32_t* out_row_map, const float* row_scale, void* workspace,
-                                 size_t workspace_bytes, int a_mode, int tile_n, const void* bias, int bias_fp32,
+                               int num_rows, const int32_t* num_rows_dev, int rows_hint, const void* weight,
+                               int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
+                               const int32_t* out_row_map, const float* row_scale, void* workspace,
+                               size_t workspace_bytes, int a_mode, int tile_n, const void* bias, int bias_fp32,
                                int few_rows_ctas, void* stream) {
   DYLLM_REQUIRE(x_rows >= 0 && in_features > 0 && out_features > 0 && num_rows >= 0, DYLLM_ERR_INVALID_ARGUMENT,
                 "gathered_linear: x_rows %d in %d out %d num_rows %d", x_rows, in_features, out_features, num_rows);

@@ -2,7 +2,7 @@
 // CTA-pair kernel of pair_gemm.cuh (one weight block per row tile), routing weight folded into the
 // down-projection epilogue, per-token sum over the top-k slots.
 //
-//   route    logits = x[idx[m]] . Wr^T (fp32), softmax over experts, top-k           (one block per row)
+//   route    logits = x[idx[m]] . Wr^T (fp32), softmax over experts, top-k       (one or four rows per block)
 //   align    (row, slot) pairs grouped by expert, row tiles of at most 256 rows  (one block)
 //   GEMM 1   h = silu(x Wg_e^T) * (x Wu_e^T) for the rows of each tile's expert
 //   GEMM 2   y[pair] = w_pair * (h Wd_e^T)

@@ -33,9 +33,10 @@
 //   gate/up   41 -> 42     43 -> 48     72 -> 52     115 -> 96    192 -> 145   355 -> 209
 //   down      31 -> 30     35 -> 34     55 -> 47     94 -> 73     174 -> 109   254 -> 136
 //   K/V       23 -> 23     25 -> 26     35 -> 31     65 -> 43     114 -> 56    177 -> 111
-// Library products of the same size: 91 against 107 us at 4096 rows, 182 against 224 at 8192 (4096 x 4096).  Few rows are
-// bound by the weight stream (4.9 of 6.5 TB/s for gate/up: an SM takes in ~50 GB/s through a stage ring whose
-// round trip spans two CTAs); many rows by the power limit (1.3 PFLOP/s at 3277 rows, as the library's products).
+// Library products of the same size: 91 against 107 us at 4096 rows, 182 against 224 at 8192 (4096 x 4096).  At 46 rows the
+// weights alone take 31, 15 and 10 us at the HBM rate (6.5 TB/s), so every product spends another 11 to 15 us beside the
+// stream (start of the ring, whose round trip spans two CTAs; partial sums; epilogue): gate/up runs at 4.8 TB/s, down at 3.4,
+// K/V at 2.9.  Many rows are bound by the power limit (1.3 PFLOP/s at 3277 rows, as the library's products).
 // Every wait is bounded; a wait that runs out raises the CTA's abort flag and the device status word.
 #pragma once
 
@@ -523,32 +524,33 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           else
             asm volatile("bar.sync 3, 128;" ::: "memory");
         }
-      } else
-      for (int c = part; c < chunks; c += 2) {
-        if (SWIGLU) {
-          uint32_t ra[32], rb[32];
-          tmem_ld_32x32(d0 + c * 32, ra);
-          tmem_ld_32x32(d0 + s.tile_n + c * 32, rb);
-          tmem_ld_wait();
-          float a[32];
-#pragma unroll
-          for (int r = 0; r < 32; ++r)
-            a[r] = silu_f(__uint_as_float(ra[r])) * __uint_as_float(rb[r]);
-          store_chunk(c, col_cta, a);
-        } else {
-#pragma unroll 1
-          for (int j = 0; j < s.nb; ++j) {
-            uint32_t ra[32];
-            tmem_ld_32x32(d0 + j * s.tile_n + c * 32, ra);
+      } else {
+        for (int c = part; c < chunks; c += 2) {
+          if (SWIGLU) {
+            uint32_t ra[32], rb[32];
+            tmem_ld_32x32(d0 + c * 32, ra);
+            tmem_ld_32x32(d0 + s.tile_n + c * 32, rb);
             tmem_ld_wait();
-            if (cut) {
-              keep_chunk(c, col_cta + j * 128, ra);
-            } else {
-              float a[32];
+            float a[32];
 #pragma unroll
-              for (int r = 0; r < 32; ++r)
-                a[r] = __uint_as_float(ra[r]);
-              store_chunk(c, col_cta + j * 128, a);
+            for (int r = 0; r < 32; ++r)
+              a[r] = silu_f(__uint_as_float(ra[r])) * __uint_as_float(rb[r]);
+            store_chunk(c, col_cta, a);
+          } else {
+#pragma unroll 1
+            for (int j = 0; j < s.nb; ++j) {
+              uint32_t ra[32];
+              tmem_ld_32x32(d0 + j * s.tile_n + c * 32, ra);
+              tmem_ld_wait();
+              if (cut) {
+                keep_chunk(c, col_cta + j * 128, ra);
+              } else {
+                float a[32];
+#pragma unroll
+                for (int r = 0; r < 32; ++r)
+                  a[r] = __uint_as_float(ra[r]);
+                store_chunk(c, col_cta + j * 128, a);
+              }
             }
           }
         }

@@ -135,7 +135,10 @@ def gathered_linear(x: torch.Tensor, weight: torch.Tensor, idx: torch.Tensor | N
     ws = _scratch(need, x.device)
     call("dyllm_gathered_linear_bias", ptr(x), x.size(0), x.size(1), x.stride(0), ptr(idx), num_rows, ptr(num_rows_dev),
          int(rows_hint), ptr(weight), n_out, ptr(out), out.stride(0), ptr(out2), out2.stride(0) if out2 is not None else 0,
-         int(split_col), ptr(out_row_map), ptr(row_scale), ptr(ws), ws.numel(), a_mode, tile_n, ptr(bias), int(bias_fp32), int(few_rows_ctas), stream_ptr(x.device))
+         int(split_col), ptr(out_row_map), ptr(row_scale), ptr(ws), ws.numel(), a_mode, tile_n, ptr(bias), int(bias_fp32),
+         int(few_rows_ctas), stream_ptr(x.device))
+    if idx is None:
+        _lib_mod.launch_count -= 1      # no row staging launch when the rows arrive packed
     return out
 
 

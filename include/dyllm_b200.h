@@ -177,11 +177,10 @@ int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ld
  * kernel on the other stream finds the remaining SMs free.  Ignored by calls that name a tile width or a_mode 1. */
 int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64_t ldx, const int32_t* idx,
                                int num_rows, const int32_t* num_rows_dev, int rows_hint, const void* weight,
-                                 int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
-                                 const int32_t* out_row_map, const float* row_scale, void* workspace,
-                                 size_t workspace_bytes, int a_mode, int tile_n, const void* bias, int bias_fp32, int few_rows_ctas,
-                                 void* stream);
-
+                               int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
+                               const int32_t* out_row_map, const float* row_scale, void* workspace,
+                               size_t workspace_bytes, int a_mode, int tile_n, const void* bias, int bias_fp32,
+                               int few_rows_ctas, void* stream);
 
 /* Bytes of workspace dyllm_swiglu_ffn needs for up to max_rows gathered rows. */
 size_t dyllm_swiglu_ffn_workspace_bytes(int max_rows, int hidden, int inter);
