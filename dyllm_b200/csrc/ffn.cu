@@ -3,8 +3,8 @@
 // built from two tcgen05 GEMMs: gate/up with the activation fused in the epilogue, then the down projection
 // whose epilogue scatters rows to their destination.  By default the rows are packed (by the caller, or by a
 // small staging copy) and run on the CTA-pair GEMM of pair_gemm.cuh, which suits every row count.  Calls that
-// name a tile width or ask for TMA gather4 run on gemm.cuh, whose launch shape follows a row-count hint.  The
-// live row count is read on the device, so no host synchronisation is needed.
+// name a tile width or ask for TMA gather4, and the sizes that use_pair() lists, run on gemm.cuh, whose launch
+// shape follows a row-count hint.  The live row count is read on the device, so no host synchronisation is needed.
 #include <atomic>
 
 #include "gemm.cuh"
@@ -127,21 +127,56 @@ void set_cut(PairGemmParams& q, int rows_hint) {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Which of the two kernels runs a call that names neither a tile width nor a_mode 1 (both give the same bits).  The pair
-// kernel needs no row estimate and wins almost everywhere; its tiles are 256 columns per pair of SMs, so narrow or short
-// products of few rows leave it with too few of them, where 64-column tiles still fill SMs (us, 64-column : pair kernel):
-//   gate/up of 1536 columns, 46 / 300 rows            30 : 35 / 31 : 47
-//   plain, 1024 columns, 46 / 100 rows                13 : 16 / 16 : 17
-//   plain, K = 1536, 4096 columns, 46 / 100 rows      12 : 14 / 15 : 17
-//   gate/up of 12288 columns, 65 .. 128 rows          43 : 48  (46 rows 41 : 42, 160 rows 70 : 50; only when the host
-//                                                     knows the count: one estimate serves every count otherwise)
-bool few_tiles(bool swiglu, int n, int K, int num_rows, const int32_t* num_rows_dev, int rows_hint) {
-  const int h = rows_hint > 0 && rows_hint < num_rows ? rows_hint : num_rows;
-  if (h > kSplitRows)
+// Which of the two kernels runs a call that names neither a tile width nor a_mode 1; both cut k into the same parts and add
+// them in the same order.  The pair kernel needs no row estimate: it suits every count that only the device knows.  Where the
+// estimate or the host's own count tells, gathered_gemm_kernel is ahead in three places (us, that kernel : pair kernel, with
+// weights from HBM):
+// * Few rows and few weights: the pair kernel's tiles are 256 columns per pair of SMs, each behind a ring whose round trip
+//   spans two CTAs; 64-column tiles, two CTAs per SM, are done sooner.
+//     1024 columns, k = 3584, 33 / 100 / 512 rows     13.1 : 15.0 / 15.6 : 16.0 / 21.8 : 21.4
+//     4096 columns, k = 1536, 33 / 100 / 256 / 300    11.3 : 13.5 / 15.3 : 17.4 / 16.5 : 18.2 / 24.8 : 16.2
+//     4096 columns, k = 2048, 33 / 100 / 200          12.2 : 14.2 / 16.6 : 18.4 / 19.0 : 20.1
+//     4096 columns, k = 4096, 33 / 100 / 200          16.9 : 19.2 / 21.1 : 22.6 / 27.0 : 27.0
+//     8192 columns, k = 4096, 33 / 200                27.0 : 25.3 / 39.4 : 35.0
+//   A count that only the device knows may be far above the estimate, where these tiles lose (4096 x 2048: 33 rows 12.4 :
+//   14.6, but 700 rows 32.7 : 25.6), so such calls take them only for the narrow and the short products.
+// * 256 x 256 tiles of a single CTA where they need no more waves than the pair kernel's tiles, as long as the weights stay
+//   in L2 (with more, the pair kernel's groups of row tiles re-read them less often):
+//     4096 columns, k = 12288, 2000 / 3000 / 8192     143 : 144 / 268 : 300 / 576 : 588
+//     4096 columns, k = 4096, 1600 / 3000 / 8192      50 : 55.6 / 99 : 108 / 203 : 213
+//     8192 columns, k = 4096, 900 / 3000 / 8192       53.7 : 57.8 / 158 : 160 / 395 : 395
+//     16384 columns, k = 4096, 2000 / 8192            225 : 211 / 837 : 785
+// * 128 x 128 tiles where one wave of them takes all rows and the pair kernel's tiles are higher than 128 rows:
+//     3584 columns, k = 3584, 513 rows 29.3 : 35.7;  5120 columns, k = 5120, 300 rows 40.1 : 47.1
+bool use_pair(int n, int K, int num_rows, const int32_t* num_rows_dev, int rows_hint) {
+  const int h = num_rows_dev && rows_hint > 0 && rows_hint < num_rows ? rows_hint : num_rows;
+  if (n <= 1024 ? h <= kSplitRows : (n <= 2048 || K <= (num_rows_dev ? 1984 : 2048)) && h <= 2 * kGemmBM)
     return false;
-  if (swiglu)
-    return !num_rows_dev && num_rows > 64 && num_rows <= 128;
-  return n <= 2048 || K < 2048;
+  if (num_rows_dev)
+    return true;
+  const int64_t weights = static_cast<int64_t>(n) * K;
+  if (h <= kGemmBM)
+    return weights > 4096 * 4096;
+  const Plan plan = make_plan(false, h, 0, n, K, 0, true, true);
+  if (plan.tile_n == 64)
+    return true;
+  const int sms = sm_count(), pairs = sms / 2;
+  int tile_n, row_tiles, waves;
+  pg_row_tiles(h, cdiv_i(h, kPgMaxRows), tile_n, row_tiles);
+  pg_lower_tiles(h, cdiv_i(n, 256), 1, pairs, tile_n, row_tiles);
+  const int blocks = pg_blocks(row_tiles, n, 1, pairs, waves);
+  if (plan.tile_n == 128)
+    return plan.tall || tile_n <= 128 || cdiv_i(h, kGemmBM) * (n / 128) > sms;
+  // a wave of 256 x 256 tiles takes as long as one of two weight blocks, 4/3 as long as one of one
+  const int own = 4 * cdiv_i(cdiv_i(h, 256) * (n / 256), sms), pair = (blocks == 2 ? 4 : 3) * waves;
+  return own > pair || (own == pair && weights > 4096 * 12288);
+}
+
+// Gate/up: 64-column tiles while the host knows that 65 to 128 rows are live and the tiles put a CTA on every SM (us for the
+// whole FFN, 64-column : pair kernel at 65 / 128 rows: 12288 columns 88 : 92 / 92 : 96, 18944 104 : 109 / 107 : 111; below,
+// 9472 74 : 74 / 78 : 77, 6144 70 : 66 / 74 : 69, 3072 59 : 55 / 64 : 59, 1536 51 : 51 / 57 : 55).
+bool use_pair_swiglu(int inter, int num_rows, const int32_t* num_rows_dev) {
+  return num_rows_dev || num_rows <= 64 || num_rows > 128 || inter / 64 <= sm_count();
 }
 
 size_t padded_rows(int rows) { return static_cast<size_t>(cdiv_i(rows, kGemmBM)) * kGemmBM; }
@@ -366,7 +401,7 @@ int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64
   g.out_row_map = out_row_map;
   g.row_scale = row_scale;
   float* partial = have_ws ? reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + stage_bytes + kTicketBytes) : nullptr;
-  if (bias || (mode == 0 && tile_n == 0 && !few_tiles(false, out_features, in_features, num_rows, num_rows_dev, rows_hint))) {
+  if (bias || (mode == 0 && tile_n == 0 && use_pair(out_features, in_features, num_rows, num_rows_dev, rows_hint))) {
     PairGemmParams q = {};
     q.m_count_dev = num_rows_dev;
     q.M = num_rows;
@@ -438,7 +473,7 @@ int dyllm_swiglu_ffn(const void* x, int x_rows, int hidden, int64_t ldx, const i
   q.partial = partial;
   const bool choose = mode == 0 && tile_n == 0;
   int rc;
-  if (choose && !few_tiles(true, inter, hidden, num_rows, num_rows_dev, rows_hint)) {
+  if (choose && use_pair_swiglu(inter, num_rows, num_rows_dev)) {
     q.K = hidden;
     q.n = inter;
     q.up_row_offset = inter;
@@ -458,7 +493,7 @@ int dyllm_swiglu_ffn(const void* x, int x_rows, int hidden, int64_t ldx, const i
   if (rc != DYLLM_OK)
     return rc;
 
-  if (choose && !few_tiles(false, hidden, inter, num_rows, num_rows_dev, rows_hint)) {
+  if (choose && use_pair(hidden, inter, num_rows, num_rows_dev, rows_hint)) {
     q.K = inter;
     q.n = hidden;
     q.up_row_offset = 0;

@@ -1,6 +1,6 @@
 // Row-gathered bf16 GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for the dense SwiGLU FFN and the K/V
-// projection of salient rows: the calls that name a tile width or TMA gather4, and products of few rows with few columns
-// (few_tiles() in ffn.cu); everything else runs on pair_gemm.cuh.
+// projection of salient rows: the calls that name a tile width or TMA gather4, and the sizes that use_pair() in ffn.cu
+// lists; everything else runs on pair_gemm.cuh.
 //
 //   D[m, n] = sum_k A[a_idx[m], k] * B[n, k]                           (fp32 accumulation in TMEM)
 //

@@ -101,6 +101,29 @@ struct PgSeg {
   int tile, part, k0, k1;
 };
 
+// Rows spread evenly over row tiles of at most kPgMaxRows, in steps of 32.
+__host__ __device__ __forceinline__ void pg_row_tiles(int m, int at_least, int& tile_n, int& row_tiles) {
+  tile_n = ((m + at_least - 1) / at_least + 31) & ~31;
+  row_tiles = (m + tile_n - 1) / tile_n;
+}
+// More and lower row tiles (the weights come from L2 the second time) give more pairs work.
+__host__ __device__ __forceinline__ void pg_lower_tiles(int m, int col_tiles, int parts, int pairs, int& tile_n,
+                                                        int& row_tiles) {
+  while (tile_n > 64 && 2 * row_tiles * col_tiles * parts <= pairs)
+    pg_row_tiles(m, 2 * row_tiles, tile_n, row_tiles);
+}
+// One or two weight blocks per CTA: two need fewer operand bytes per flop, one gives twice the tiles to fill the waves
+// with.  A wave of one-block tiles takes 2/3 to 3/4 of the time of a wave of two-block tiles at 256 rows (62 B/clk of
+// operands against 47), and half at few rows.  (K = 12288, 4096 columns: 5000 rows 600 us in five waves of one block, 450 us
+// in three of two; 3277 rows three against two waves, which is even.)
+__host__ __device__ __forceinline__ int pg_blocks(int row_tiles, int n, int parts, int pairs, int& waves) {
+  const int w1 = (row_tiles * ((n + 255) >> 8) * parts + pairs - 1) / pairs;
+  const int w2 = (row_tiles * ((n + 511) >> 9) * parts + pairs - 1) / pairs;
+  const int nb = w1 * 2 <= w2 * 3 ? 1 : 2;
+  waves = nb == 1 ? w1 : w2;
+  return nb;
+}
+
 __device__ __forceinline__ bool pg_schedule(const PairGemmParams& p, bool swiglu, PgSched& s) {
   s.pairs = gridDim.x >> 1;
   s.pair = blockIdx.x >> 1;
@@ -111,10 +134,9 @@ __device__ __forceinline__ bool pg_schedule(const PairGemmParams& p, bool swiglu
     s.tile_n = (min(p.tiles_dev[1], kPgMaxRows) + 31) & ~31;
   } else {
     s.m = p.m_count_dev ? min(*p.m_count_dev, p.M) : p.M;
-    s.row_tiles = (s.m + kPgMaxRows - 1) / kPgMaxRows;
-    // rows spread evenly over the tiles, in steps of 32
-    s.tile_n = s.row_tiles ? ((s.m + s.row_tiles - 1) / s.row_tiles + 31) & ~31 : 32;
-    s.row_tiles = (s.m + s.tile_n - 1) / s.tile_n;
+    if (s.m <= 0)
+      return false;
+    pg_row_tiles(s.m, (s.m + kPgMaxRows - 1) / kPgMaxRows, s.tile_n, s.row_tiles);
   }
   if (s.row_tiles <= 0)
     return false;
@@ -128,20 +150,11 @@ __device__ __forceinline__ bool pg_schedule(const PairGemmParams& p, bool swiglu
   if (!swiglu && !p.row_tiles && p.partial && p.max_parts > 1 && s.m <= kSplitRows)
     s.parts = effective_splits((s.m + kGemmBM - 1) / kGemmBM, p.cut_col_tiles, p.cut_slots, p.max_parts, s.kt);
   s.part_kt = (s.kt + s.parts - 1) / s.parts;
-  // More and lower row tiles (the weights come from L2 the second time) give more pairs work, too.
   if (!p.row_tiles)
-    while (s.tile_n > 64 && 2 * s.row_tiles * ((p.n + pair_cols - 1) / pair_cols) * s.parts <= s.pairs) {
-      const int more = 2 * s.row_tiles;
-      s.tile_n = ((s.m + more - 1) / more + 31) & ~31;
-      s.row_tiles = (s.m + s.tile_n - 1) / s.tile_n;
-    }
-  // One or two weight blocks per CTA: two need fewer operand bytes per flop, one gives twice the tiles to fill the waves
-  // with.  A wave of one-block tiles takes ~2/3 of the time of a wave of two-block tiles at 256 rows (62 B/clk of operands
-  // against 47), and half at few rows.  (K = 12288, 4096 columns: 5000 rows 600 us in five waves of one block, 450 us in
-  // three of two; 3277 rows three against two waves, which is even.)
-  const int t1 = s.row_tiles * ((p.n + 255) >> 8), t2 = s.row_tiles * ((p.n + 511) >> 9);
-  const int w1 = (t1 * s.parts + s.pairs - 1) / s.pairs, w2 = (t2 * s.parts + s.pairs - 1) / s.pairs;
-  s.nb = swiglu ? (s.narrow ? 1 : 2) : (p.row_tiles ? (s.tile_n > 128 ? 2 : 1) : (w1 * 2 <= w2 * 3 ? 1 : 2));
+    pg_lower_tiles(s.m, (p.n + pair_cols - 1) / pair_cols, s.parts, s.pairs, s.tile_n, s.row_tiles);
+  int waves;
+  s.nb = swiglu ? (s.narrow ? 1 : 2)
+                : p.row_tiles ? (s.tile_n > 128 ? 2 : 1) : pg_blocks(s.row_tiles, p.n, s.parts, s.pairs, waves);
   const int cols = swiglu ? pair_cols : s.nb * 256;
   s.col_tiles = (p.n + cols - 1) / cols;
   s.units = s.row_tiles * s.col_tiles * s.parts;

@@ -53,3 +53,20 @@ def test_both_kernels_cut_alike(cuda_device, k, n, hint):
         # one bf16 rounding (2^-9 of a value at most) of an fp32 sum
         assert ((got[:live].double() - ref).norm() / ref.norm()).item() <= 2.0 ** -8
     assert _lib.load().dyllm_device_status() == 0
+
+
+@pytest.mark.parametrize("k,n", [(2048, 4096), (4096, 4096), (3584, 3584), (1536, 4096), (3584, 1024), (4096, 2048)])
+def test_chosen_kernel_gives_the_pair_kernels_bits(cuda_device, k, n):
+    """Counts on both sides of the lines at which the host's own count changes the kernel (64-column tiles, the pair kernel,
+    one wave of 128 x 128 tiles, 256 x 256 tiles)."""
+    from dyllm_b200 import _lib, ops
+
+    g = torch.Generator(device="cuda").manual_seed(k + n)
+    x = torch.randn(3000, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(n, k, generator=g, device="cuda") * 0.05).bfloat16()
+    zero = torch.zeros(n, dtype=torch.bfloat16, device="cuda")
+    for rows in (1, 64, 128, 129, 256, 257, 384, 512, 513, 900, 1600, 3000):
+        got = ops.gathered_linear(x, w, num_rows=rows)
+        want = ops.gathered_linear(x, w, num_rows=rows, bias=zero, bias_fp32=True)
+        assert torch.equal(got, want), f"{rows} rows"
+    assert _lib.load().dyllm_device_status() == 0
