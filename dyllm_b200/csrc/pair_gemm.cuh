@@ -153,8 +153,10 @@ __device__ __forceinline__ bool pg_schedule(const PairGemmParams& p, bool swiglu
   if (!p.row_tiles)
     pg_lower_tiles(s.m, (p.n + pair_cols - 1) / pair_cols, s.parts, s.pairs, s.tile_n, s.row_tiles);
   int waves;
+  // grouped tiles up to 128 rows high: one block; higher ones by the waves, too (8 experts of 200 rows each, 2048 columns: 32
+  // tiles of two blocks leave more than half of the pairs idle)
   s.nb = swiglu ? (s.narrow ? 1 : 2)
-                : p.row_tiles ? (s.tile_n > 128 ? 2 : 1) : pg_blocks(s.row_tiles, p.n, s.parts, s.pairs, waves);
+                : p.row_tiles && s.tile_n <= 128 ? 1 : pg_blocks(s.row_tiles, p.n, s.parts, s.pairs, waves);
   const int cols = swiglu ? pair_cols : s.nb * 256;
   s.col_tiles = (p.n + cols - 1) / cols;
   s.units = s.row_tiles * s.col_tiles * s.parts;

@@ -87,7 +87,7 @@ def test_device_count_column_split_and_fewer_ctas(cuda_device, live, ctas):
     assert bool((out[live:] == 5.0).all()) and bool((out2[live:] == 5.0).all())
 
 
-@pytest.mark.parametrize("rows,experts,top_k,skew", [(1, 8, 2, 0), (33, 64, 8, 0), (300, 8, 1, 1), (700, 16, 4, 1), (1500, 4, 2, 2)])
+@pytest.mark.parametrize("rows,experts,top_k,skew", [(200, 8, 8, 0), (1, 8, 2, 0), (33, 64, 8, 0), (300, 8, 1, 1), (700, 16, 4, 1), (1500, 4, 2, 2)])
 def test_grouped_experts(cuda_device, rows, experts, top_k, skew):
     """Experts without rows, with a few, and with several row tiles."""
     from dyllm_b200 import ops
