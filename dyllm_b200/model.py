@@ -151,6 +151,28 @@ def _kv_overlap() -> bool:
     return os.environ.get("DYLLM_KV_OVERLAP", "1") != "0" and layers._projection_backend != "tcgen05"
 
 
+# Query projections of up to this many rows are launched after the K/V branch.
+_KV_FIRST_ROWS = 256
+_sm_counts: dict = {}
+
+
+def _kv_ctas(rows: int, columns: int, device) -> int:
+    """SMs for the salient rows' K/V product beside a query projection of ``rows`` x ``columns`` (0: all of them).
+
+    The library kernel runs tiles of 256 x 256, one per SM at a time.  Where its last wave, one of several, leaves 32 to 80
+    of 148 SMs idle, the product keeps to those and the weights stream in under the projection; more idle SMs or fewer
+    need no rule, and with a single wave the library takes other tiles.  Both branches of a layer, us, 32 salient rows,
+    K/V on these SMs : on all (4096 -> 4096 + 8192): 4096 rows (40 idle) 102 : 111, 6144 (60) 153 : 155 (200 salient rows
+    160 : 169), 8192 (80) 192 : 191 (199 : 211); not so 2560 (136 idle) 96 : 88, 4608 (8) 132 : 116, 2048 (one wave) 86 : 72.
+    At 2048 -> 2048 + 4096 and 8192 rows (40 idle) 52 : 59, but 72 : 66 with 200 salient rows."""
+    sms = _sm_counts.get(device)
+    if sms is None:
+        sms = _sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
+    tiles = -(-rows // 256) * -(-columns // 256)
+    idle = -tiles % sms
+    return idle if tiles > sms and 32 <= idle <= 80 else 0
+
+
 def _forward_sparse_overlapped(self, positions, hidden_states, salient_rows):
     ctx, md = get_context(), get_metadata()
     H, Hkv, D = self.num_heads, self.num_kv_heads, self.head_dim
@@ -166,24 +188,37 @@ def _forward_sparse_overlapped(self, positions, hidden_states, salient_rows):
     v_new = torch.empty((cap, self.kv_size), dtype=hidden_states.dtype, device=dev)
     dv = torch.empty((cap, Hkv, D), dtype=hidden_states.dtype, device=dev)
     rows_k = ctx.idx_salient_row_k if ctx.idx_salient_row_k is not None else ctx.idx_salient_row
-    # The query projection is launched first: it fills the SMs, and what its last wave leaves idle is where the other
-    # branch belongs.  (The other way round that branch takes SMs from the first wave, which then needs one wave more.)
+    rows = hidden_states.size(0)
+    kw = {}
+    if as_defined(self.kv_proj, ColumnParallelLinear, "forward_gathered"):
+        ctas = _kv_ctas(rows, self.q_size, dev)
+        if ctas:
+            kw["few_rows_ctas"] = ctas
+
+    def kv_branch():
+        with torch.cuda.stream(side):
+            self.kv_proj.forward_gathered(salient_rows, None, cap, n_dev, hint, split_col=self.kv_size, out=(k_new, v_new),
+                                          **kw)
+            k3 = k_new.view(cap, Hkv, D)
+            if self.k_norm is not None:
+                k3 = self.k_norm.forward_heads_(k3, n_dev)
+            ops.kv_cache_update(k3, v_new.view(cap, Hkv, D), rows_k, positions, ctx.idx_salient_row,
+                                self.rotary_emb.cos_sin_cache.view(-1, D), ctx.cu_seqlens_k, self.k_cache.seq_start_gpu,
+                                self.attn.v_cache.seq_start_gpu, md.running_seqs_tensor, self.k_cache.cache,
+                                self.attn.v_cache.cache, n_dev, dv=dv)
+
+    # A query projection of many rows is launched first: it fills the SMs, and what its last wave leaves idle is where the
+    # other branch belongs.  (The other way round that branch takes SMs from the first wave, which then needs one wave more:
+    # 2048 rows 96 against 72 us for both.)  One of few rows is the shorter branch, so the other one gets the SMs first
+    # (a batch of one sequence: 6890 against 6960 us per eight steps of four layers).
     forked = main.record_event()
-    q = self.q_proj(hidden_states).view(-1, H, D)
     side.wait_event(forked)
-    # Beside a query projection of many rows the few salient rows' product keeps to 40 SMs, about what the library
-    # kernel's last wave leaves idle: the weights stream in under it either way.  A short one has no such tail.
-    ctas = 40 if hidden_states.size(0) >= 2048 and as_defined(self.kv_proj, ColumnParallelLinear, "forward_gathered") else 0
-    with torch.cuda.stream(side):
-        self.kv_proj.forward_gathered(salient_rows, None, cap, n_dev, hint, split_col=self.kv_size, out=(k_new, v_new),
-                                      **({"few_rows_ctas": ctas} if ctas else {}))
-        k3 = k_new.view(cap, Hkv, D)
-        if self.k_norm is not None:
-            k3 = self.k_norm.forward_heads_(k3, n_dev)
-        ops.kv_cache_update(k3, v_new.view(cap, Hkv, D), rows_k, positions, ctx.idx_salient_row,
-                            self.rotary_emb.cos_sin_cache.view(-1, D), ctx.cu_seqlens_k, self.k_cache.seq_start_gpu,
-                            self.attn.v_cache.seq_start_gpu, md.running_seqs_tensor, self.k_cache.cache,
-                            self.attn.v_cache.cache, n_dev, dv=dv)
+    if rows <= _KV_FIRST_ROWS:
+        kv_branch()
+        q = self.q_proj(hidden_states).view(-1, H, D)
+    else:
+        q = self.q_proj(hidden_states).view(-1, H, D)
+        kv_branch()
     q = _norm_and_rotate(self.rotary_emb, positions, q, self.q_norm)
     main.wait_stream(side)
     k_full = self.k_cache.get_seqs(md.running_seqs_tensor, allow_view=True, seq_ids_list=md.running_seqs)
