@@ -693,7 +693,6 @@ class Attention(nn.Module):
         self.context_cache = CacheManager(self.num_heads * self.head_dim)
         self.v_cache = CacheManager(self.num_kv_heads * self.head_dim)
         self._hint_host = None      # pinned int32[1]: this layer's salient count, copied back without waiting
-        self._hint_event = None
         self._hint = 0
 
     def _next_hint(self, count_dev: torch.Tensor, capacity: int, fixed: int = 0) -> int:
@@ -705,15 +704,15 @@ class Attention(nn.Module):
         if fixed:
             return min(fixed, capacity)
         if self._hint_host is None:
-            self._hint_host = torch.zeros(1, dtype=torch.int32).pin_memory()
-            self._hint_event = torch.cuda.Event()
-        elif self._hint_event.query():
-            self._hint = int(self._hint_host[0])
-            profiling.count("salient_rows", self._hint)
+            self._hint_host = torch.empty(1, dtype=torch.int32).pin_memory()
         else:
-            return min(self._hint, capacity) if self._hint else capacity
+            arrived = self._hint_host.item()
+            if arrived < 0:
+                return min(self._hint, capacity) if self._hint else capacity
+            self._hint = arrived
+            profiling.count("salient_rows", arrived)
+        self._hint_host.fill_(-1)            # no count: until the copy has arrived
         self._hint_host.copy_(count_dev, non_blocking=True)
-        self._hint_event.record()
         return min(self._hint, capacity) if self._hint else capacity
 
     def forward(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, dv: torch.Tensor | None = None) -> torch.Tensor:
