@@ -197,7 +197,8 @@ class StepRunner:
         self.salient_counts: list[int] = []
         self.use_graphs = use_graphs
         # salient-row estimate baked into the launches of a captured step (any value is correct; it decides whether
-        # products with few columns take 64-column tiles, everything else follows the count on the device)
+        # products with few columns take 64-column tiles and into how many parts few rows' products are cut along k,
+        # everything else follows the count on the device)
         self.graph_rows_hint = max(1, int(graph_rows_hint))
         # With several ranks a step is captured whole, NCCL all-reduces and peer-memory exchanges included
         # (DYLLM_TP_GRAPHS=whole, the default).  NCCL keeps a communicator alive for as long as a graph that
