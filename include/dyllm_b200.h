@@ -170,11 +170,12 @@ int dyllm_gathered_linear(const void* x, int x_rows, int in_features, int64_t ld
                           int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
                           const int32_t* out_row_map, const float* row_scale, void* workspace,
                           size_t workspace_bytes, int a_mode, int tile_n, void* stream);
-/* The same call with three more arguments.  bias (bf16 [out_features], 2-byte aligned, nullable) is added to the fp32 sum before the scale
- * and the one rounding (bias_fp32 = 1), or to the bf16 result with a rounding of its own, as a separate addition has it
- * (bias_fp32 = 0); only with a_mode <= 0 and tile_n 0.  few_rows_ctas serves a stream that runs beside another one: while
- * all live rows fit one row tile (256 rows) the product keeps to `few_rows_ctas` CTAs (one per SM; 0 = all SMs), so that a
- * kernel on the other stream finds the remaining SMs free.  Ignored by calls that name a tile width or a_mode 1. */
+/* The same call with three more arguments.  bias (bf16 [out_features], 2-byte aligned, nullable) is added to the fp32 sum
+ * before the scale and the one rounding (bias_fp32 = 1), or to the bf16 result with a rounding of its own, as a separate
+ * addition has it (bias_fp32 = 0); only with a_mode <= 0 and tile_n 0.  few_rows_ctas serves a stream that runs beside
+ * another one: while all live rows fit one row tile (256 rows) the CTA-pair kernel keeps to `few_rows_ctas` CTAs (one per
+ * SM; 0 = all SMs), so that a kernel on the other stream finds the remaining SMs free.  Products with few columns or a short
+ * k, and calls that name a tile width or a_mode 1, run on another kernel, which ignores it. */
 int dyllm_gathered_linear_bias(const void* x, int x_rows, int in_features, int64_t ldx, const int32_t* idx,
                                int num_rows, const int32_t* num_rows_dev, int rows_hint, const void* weight,
                                int out_features, void* out, int64_t ldo, void* out2, int64_t ldo2, int split_col,
